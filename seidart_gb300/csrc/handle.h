@@ -65,7 +65,7 @@ struct Layout {
   int P, NX, NY, NZ, W, ysplit, nslots;
   size_t fsz;  // floats per field
   size_t off_ctl, off_fields, off_mem[18], mem_sz[18], off_fieldsB, off_memB[18], off_coef, coef_plane, off_axis[3],
-      off_q3, off_src, off_rec, off_traces, off_slots, off_res, total;
+      off_q3, off_src, off_rec, off_traces, off_slots, off_res, off_words, total;
 };
 
 }  // namespace sfd
@@ -94,8 +94,8 @@ struct sfd_handle_s {
   sfd::Seis2Step s2s[2];
   sfd::Launch launch1;       // single-pass geometry
   int res_state = 0;    // on-chip runs: 0 not yet checked, 1 usable, -1 not usable
-  sfd::ResPlan res_plan;     // electromag2
-  sfd::ResPlan res_plan_adj;  // electromag2, the adjoint sweep's (no three-row tiles)
+  sfd::Em2Plan res_plan;     // electromag2
+  sfd::ResPlan res_plan_adj;  // electromag2, the adjoint sweep's
   sfd::Seis2ResPlan s2_plan;  // seismic2
   int64_t step = 0;
   unsigned long long wait_ns = sfd::kDefaultWaitNs;  // longest wait of an on-chip run for a neighbouring tile
@@ -156,8 +156,14 @@ struct sfd_handle_s {
 namespace sfd {
 
 // Starts a run at `step` on the handle's stream: the control block's step
-// base and error word, the norm slots cleared.
-void begin_run(sfd_handle_s* h, int64_t step);
+// base and error word, the norm slots cleared, the hand-over tags of an
+// on-chip run counted on by `hand_overs`.
+void begin_run(sfd_handle_s* h, int64_t step, int hand_overs = 0);
+// The tiling of an electromag2 handle's adjoint sweep for the current device.
+bool adjoint_plan(sfd_handle_s* h);
+// Counts the hand-over tags on for an on-chip run inside an adjoint segment
+// (the error word and the norms stay).
+void count_hand_overs(sfd_handle_s* h, int hand_overs);
 // The run's largest field norm from the per-block slots into the control block.
 void reduce_norms(sfd_handle_s* h);
 // Whether this handle's runs go on chip (decided once per handle).

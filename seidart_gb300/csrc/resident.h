@@ -18,25 +18,25 @@ namespace sfd {
 constexpr int kResMaxTiles1D = 32;
 // Largest number of tiles (CTAs, at most one per SM) of one on-chip run.
 constexpr int kResMaxTiles = 256;
-// Threads of a CTA: up to 15 warps own the cells (four cells of kResRows
-// rows per thread, kResRows3 in interior electromag2 tiles), the last warp
-// moves the tile's edges to and from the neighbouring tiles.
+// Threads of a CTA of the electromag2 adjoint sweep: up to 15 warps own the
+// cells (four cells of kResRows rows per thread), the last warp moves the
+// tile's edges to and from the neighbouring tiles.
 constexpr int kResThreads = 512;
 constexpr int kResCellThreads = kResThreads - 32;
 constexpr int kResRows = 2;
-// Rows per thread in an electromag2 tile of interior cells only (no CPML
-// strip, no Dirichlet plane), whose cells all take the short update: the
-// planner gives such tiles more cells than the others, so that the tiles
-// with the longer strip and boundary updates can be made smaller.
-constexpr int kResRows3 = 3;
+// The electromag2 runs' tiles (em2_tile.cuh): cells of halo on a side with a
+// neighbour, which is also the number of steps between two hand-overs; the
+// most frame rows a warp holds, and the most warps of a CTA.
+constexpr int kTileHalo = 4;
+constexpr int kEm2MaxRows = 4;
+constexpr int kEm2MaxWarps = 16;
 // Receivers a CTA lists in shared memory; a tile holding more scans the
 // whole receiver list every step instead.
 constexpr int kResMaxLocalRec = 256;
 
-// Tiling of one on-chip run: ntz tile rows, each cut into its own tiles.
+// Tiling of one adjoint sweep: ntz tile rows, each cut into its own tiles.
 // tile[b] packs x0 | x1 << 16, z0 | z1 << 16, row | (index in row) << 16 and
-// the tile count of its row | (interior tile: kResRows3 rows per thread) << 16;
-// column bounds are multiples of 4 (except NX).
+// the tile count of its row; column bounds are multiples of 4 (except NX).
 // Tiles that hold CPML strip or boundary cells take the longer update and are
 // made smaller.
 struct ResPlan {
@@ -44,6 +44,33 @@ struct ResPlan {
   int4 tile[kResMaxTiles];
   size_t smem;  // dynamic shared memory of the largest tile
 };
+
+// Tiling of one electromag2 run: tile columns of about equal width, each cut
+// into its own bands (at most ntz).  tile[b] packs the owned cells, x0 | x1 <<
+// 16 and z0 | z1 << 16 (column bounds are multiples of 4 except NX), and
+// whether the frame holds strip or boundary cells (1) and x-strip ones (2).  A CTA has `warps` warps of
+// rb frame rows.
+struct Em2Plan {
+  int ntiles, ntz, rb, warps;
+  int4 tile[kResMaxTiles];
+  size_t smem;  // dynamic shared memory of the largest tile
+};
+
+// Hand-over words of an electromag2 run (resident2d.cu) inside the handle's
+// state buffer, two copies, each: {Ex, Ez, Hy, tag} by cell [NZ][P], {dEx_dz,
+// dHy_dz, -, tag} by z-strip cell [2W][P] and {dEz_dx, dHy_dx, -, tag} by
+// x-strip cell [NZ][2W].
+inline size_t em2_word_bytes(int P, int NZ, int W) {
+  return 2 * sizeof(uint4) * ((size_t)NZ * P + 2 * (size_t)W * P + (size_t)NZ * 2 * W);
+}
+// Largest grid (cells of pitch) an electromag2 run can hold on chip; larger
+// ones get no hand-over words.
+constexpr size_t kEm2MaxCells = (size_t)kResMaxTiles * 124 * kEm2MaxRows * kEm2MaxWarps;
+// Hand-overs of a run of nsteps steps: after every kTileHalo-th but the last;
+// a run of no more steps has one before its first.
+__host__ __device__ inline int em2_hand_overs(int nsteps) {
+  return nsteps <= kTileHalo ? 1 : (nsteps - 1) / kTileHalo;
+}
 
 // Edge arrays inside a handle's state buffer.  Every edge value travels as
 // one 8-byte word {value, tag}, the tag being one more than the step that
@@ -100,11 +127,11 @@ struct Em2Resident {
   AxisTab X, Z;
   float dbH;
   IoArgs io;
-  ResPlan plan;
-  ResScratch r;
+  Em2Plan plan;
+  uint4* words;
   int t0, nsteps;
   unsigned long long limit_ns;  // longest wait for a neighbour before the run is abandoned
-  unsigned tag_bias;            // added to every awaited edge tag; 0 except in the timeout test aid
+  unsigned tag_bias;            // added to every awaited tag; 0 except in the timeout test aid
   ResDump dump;
   // checkpoints: after every ckpt_every-th step of the run (not its last),
   // the state in the sfd_checkpoint_save layout at ckpt.base + (s / every) * stride
@@ -183,17 +210,15 @@ cudaError_t seis2_resident_launch(const Seis2Resident& a, cudaStream_t s);
 
 // Pick the tiling of an NX x NZ electromag2 grid with npml-cell strips for
 // `max_ctas` CTAs of at most `max_smem` bytes of shared memory.  Returns
-// false when the grid does not fit on chip.  rows3: tiles of interior cells
-// may take kResRows3 rows per thread (the forward kernel's plans; the adjoint
-// sweep's tiles all take kResRows).
-bool em2_resident_plan(int NX, int NZ, int npml, int max_ctas, size_t max_smem, ResPlan* out, bool rows3);
-// Dynamic shared memory of a TW x TZ tile with RB rows per thread.
-size_t em2_resident_smem(int TW, int TZ, int RB);
-// Set the kernel's shared-memory limit (once per device) and return how many
-// CTAs of `smem` bytes fit on one SM.
-cudaError_t em2_resident_prepare(const ResPlan& plan, int* ctas_per_sm);
+// false when the grid does not fit on chip.
+bool em2_resident_plan(int NX, int NZ, int npml, int max_ctas, size_t max_smem, Em2Plan* out);
+// Set the kernels' shared-memory limit (once per device) and return how many
+// CTAs of the plan fit on one SM.
+cudaError_t em2_resident_prepare(const Em2Plan& plan, int* ctas_per_sm);
 cudaError_t em2_resident_launch(const Em2Resident& a, cudaStream_t s);
 
+// The same for the adjoint sweep's tiles.
+bool em2_adj_resident_plan(int NX, int NZ, int npml, int max_ctas, size_t max_smem, ResPlan* out);
 // The adjoint sweep's dynamic shared memory for the largest tile of `plan`
 // on an NX x NZ grid with W-cell strips; its set-up for `plan` (the kernel's
 // shared-memory limit, once per device; how many CTAs fit on one SM, 0 when

@@ -34,6 +34,7 @@
 // with cp.async while it runs phase B, and prefetches the strips' psi' into
 // L2.
 #include <algorithm>
+#include <vector>
 
 #include "resident_common.cuh"
 
@@ -804,7 +805,122 @@ __global__ void __launch_bounds__(kResThreads, 1) em2_adj_resident_kernel(const 
   }
 }
 
+// Cost model of the planner, in four-cell groups: a group in a CPML strip or
+// on a boundary plane takes the longer update, this many times an interior
+// group's (weights 2 to 8 changed the sweep of the 1040 x 540 grid by under
+// 1 %); a build-time tunable.
+#ifndef SFD_RES_ADJ_GENERAL_COST
+#define SFD_RES_ADJ_GENERAL_COST 4.0
+#endif
+
+// Cut n items of weight 1 + beta * gen[q] into `parts` runs of about equal
+// weight; bounds[0] = 0, bounds[parts] = n.  False if a run would be empty.
+bool cut_weighted(int n, const std::vector<int>& gen, double beta, int parts, int* bounds) {
+  std::vector<double> acc(n + 1, 0.0);
+  for (int q = 0; q < n; ++q) acc[q + 1] = acc[q] + 1.0 + beta * gen[q];
+  bounds[0] = 0;
+  int q = 0;
+  for (int c = 1; c < parts; ++c) {
+    const double target = acc[n] * c / parts;
+    while (q < n && acc[q] < target) ++q;
+    q = std::max(q, bounds[c - 1] + 1);
+    if (q > n - (parts - c)) return false;
+    bounds[c] = q;
+  }
+  bounds[parts] = n;
+  return true;
+}
+
 }  // namespace
+
+bool em2_adj_resident_plan(int NX, int NZ, int npml, int max_ctas, size_t max_smem, ResPlan* out) {
+  const int W = npml;
+  const double kGeneralCost = SFD_RES_ADJ_GENERAL_COST;
+  const int ng = (NX + 3) / 4;  // four-cell column groups
+  std::vector<int> gcol(ng), grow(NZ);
+  for (int g = 0; g < ng; ++g) {
+    int gen = 4 * g + 3 >= NX ? 1 : 0;
+    for (int i = 4 * g; i < std::min(NX, 4 * g + 4); ++i) gen |= (i < W || i >= NX - W || i < 1 || i > NX - 3) ? 1 : 0;
+    gcol[g] = gen;
+  }
+  for (int k = 0; k < NZ; ++k) grow[k] = (k < W || k >= NZ - W || k < 1 || k > NZ - 3) ? 1 : 0;
+  std::vector<int> pr(NZ + 1, 0);
+  for (int k = 0; k < NZ; ++k) pr[k + 1] = pr[k] + grow[k];
+  max_ctas = std::min(max_ctas, kResMaxTiles);
+
+  // Whether a tile of ngp groups and nr rows fits one CTA.
+  auto fits = [&](int ngp, int nr) {
+    const int tyt = (nr + kResRows - 1) / kResRows;
+    return ngp * tyt <= kResCellThreads && 4 * ngp + nr <= 32 * kResFetchPerLane &&
+           sizeof(float) * (32 * (size_t)kResRows * kResCellThreads + 8 * (size_t)(tyt + 1) * ngp + 2 * (size_t)nr * (ngp + 1)) <=
+               max_smem;
+  };
+  // Cut tile row [z0, z1) into tiles of cost <= C, greedily from the left;
+  // returns the tile count (or a count above max_ctas if impossible) and
+  // the group bounds in `cuts`.
+  auto cut_row = [&](int z0, int z1, double C, std::vector<int>* cuts) {
+    const int nr = z1 - z0, gr = pr[z1] - pr[z0];
+    int count = 0, g0 = 0;
+    double cost = 0.0;
+    if (cuts) cuts->assign(1, 0);
+    for (int g = 0; g < ng; ++g) {
+      const double cg = gcol[g] ? kGeneralCost * nr : gr * kGeneralCost + (nr - gr);
+      if (g > g0 && (cost + cg + 1.0 + nr > C || !fits(g - g0 + 1, nr))) {
+        ++count;
+        if (cuts) cuts->push_back(g);
+        g0 = g;
+        cost = 0.0;
+      }
+      if (!fits(g - g0 + 1, nr) || cg + 1.0 + nr > C) return max_ctas + 1;  // one group alone does not fit
+      cost += cg + 1.0;
+    }
+    ++count;
+    if (cuts) cuts->push_back(ng);
+    return count > kResMaxTiles1D ? max_ctas + 1 : count;
+  };
+
+  const double betas[] = {0.0, 1.0, 2.0, 3.0, 5.0, 8.0};
+  double best = 0.0;
+  bool found = false;
+  int best_rows[kResMaxTiles1D + 1], best_ntz = 0;
+  int rb[kResMaxTiles1D + 1];
+  for (int ntz = 1; ntz <= std::min(kResMaxTiles1D, NZ); ++ntz) {
+    for (double bzw : betas) {
+      if (!cut_weighted(NZ, grow, bzw, ntz, rb)) continue;
+      double lo = 0.0, hi = 1e12;
+      auto tiles_at = [&](double C) {
+        int total = 0;
+        for (int r = 0; r < ntz && total <= max_ctas; ++r) total += cut_row(rb[r], rb[r + 1], C, nullptr);
+        return total;
+      };
+      if (tiles_at(hi) > max_ctas) continue;
+      for (int it = 0; it < 40 && hi - lo > 0.5; ++it) {
+        const double mid = 0.5 * (lo + hi);
+        (tiles_at(mid) <= max_ctas ? hi : lo) = mid;
+      }
+      if (!found || hi < best * (1.0 - 1e-9)) {
+        best = hi;
+        found = true;
+        best_ntz = ntz;
+        for (int r = 0; r <= ntz; ++r) best_rows[r] = rb[r];
+      }
+    }
+  }
+  if (!found) return false;
+  out->ntz = best_ntz;
+  out->ntiles = 0;
+  out->smem = 0;
+  std::vector<int> cuts;
+  for (int r = 0; r < best_ntz; ++r) {
+    const int z0 = best_rows[r], z1 = best_rows[r + 1];
+    const int n = cut_row(z0, z1, best, &cuts);
+    for (int c = 0; c < n; ++c) {
+      const int x0 = 4 * cuts[c], x1 = std::min(NX, 4 * cuts[c + 1]);
+      out->tile[out->ntiles++] = make_int4(x0 | (x1 << 16), z0 | (z1 << 16), r | (c << 16), n);
+    }
+  }
+  return true;
+}
 
 size_t em2_adj_resident_smem(const ResPlan& plan, int NX, int NZ, int W) {
   size_t m = 0;

@@ -66,7 +66,7 @@ AdjState adj_state_at(const AdjLayout& A, char* base) {
 bool adjoint_on_chip(sfd_handle* h) {
   if (h->adj_res_state) return h->adj_res_state > 0;
   h->adj_res_state = -1;
-  if (!resident_usable(h)) return false;
+  if (!resident_usable(h) || !adjoint_plan(h)) return false;
   int per_sm = 0;
   if (em2_adj_resident_prepare(h->res_plan_adj, h->cfg.nx, h->cfg.nz, h->L.W, &per_sm) != cudaSuccess || per_sm < 1) {
     cudaGetLastError();
@@ -422,8 +422,7 @@ int32_t sfd_run_checkpointed(sfd_handle* h, int64_t nsteps, void* dev_ckpt, size
   if (h->cfg.kind == SFD_ELECTROMAG2 && resident_usable(h)) {
     // one launch for the whole run, the checkpoints written from chip
     const Layout& L = h->L;
-    begin_run(h, h->step);
-    CK(cudaMemsetAsync(h->base + L.off_res, 0, res_scratch_bytes(L.P, L.NZ, res_edge_fields(h->cfg.kind)), h->stream));
+    begin_run(h, h->step, em2_hand_overs((int)nsteps));
     Em2Resident ra = resident_args(h, nsteps);
     ra.ckpt.base = base;
     ra.ckpt.stride = stride;
@@ -530,7 +529,6 @@ static int em2_adjoint_sweep_on_chip(sfd_handle* h, const AdjLayout& A, int64_t 
   const Layout& L = h->L;
   const AdjState Lc = adj_state_at(A, h->adj + A.lam[h->adj_cur]);
   const Em2Args& e = h->em2;
-  const Em2Resident fr = resident_args(h, nsteps);
   Em2AdjResident ar;
   ar.NX = h->cfg.nx; ar.NZ = h->cfg.nz; ar.P = L.P; ar.W = L.W;
   ar.Lx = Lc.Ex; ar.Lz = Lc.Ez; ar.Lh = Lc.Hy; ar.LA = Lc.A; ar.LB = Lc.B; ar.LC = Lc.C; ar.LD = Lc.D;
@@ -549,8 +547,10 @@ static int em2_adjoint_sweep_on_chip(sfd_handle* h, const AdjLayout& A, int64_t 
   ar.nsteps = (int)nsteps;
   ar.ctl = (Ctl*)(h->base + L.off_ctl);
   ar.plan = h->res_plan_adj;
-  ar.r = fr.r;
-  ar.limit_ns = fr.limit_ns;
+  ar.r.erow = (uint2*)(h->base + L.off_res);
+  ar.r.NZp = res_nzp(h->cfg.nz);
+  ar.r.ecol = ar.r.erow + 4 * kResMaxTiles1D * (size_t)L.P;
+  ar.limit_ns = h->wait_ns;
   CK(cudaMemsetAsync(h->base + L.off_res, 0, res_scratch_bytes(L.P, L.NZ), h->stream));
   CK(em2_adj_resident_launch(ar, h->stream));
   CK(cudaGetLastError());
@@ -598,8 +598,7 @@ int32_t sfd_adjoint_record(sfd_handle* h, int64_t nsteps) {
   const Layout& L = h->L;
   r = em2_save_slot0(h, A);
   if (r) return r;
-  begin_run(h, h->step);
-  CK(cudaMemsetAsync(h->base + L.off_res, 0, res_scratch_bytes(L.P, L.NZ), h->stream));
+  begin_run(h, h->step, em2_hand_overs((int)nsteps));
   const Em2Resident own = resident_args(h, nsteps);
   CK(em2_resident_launch(em2_dump_args(h, A, h->step, nsteps), h->stream));  // receivers recorded as in sfd_run
   reduce_norms(h);
@@ -645,7 +644,7 @@ int32_t sfd_adjoint_segment(sfd_handle* h, int64_t nsteps) {
     // forward recompute on chip: slot s + 1 <- the state after step s0 + s
     Em2Resident fr = em2_dump_args(h, A, s0, nsteps);
     fr.io.nrec = 0;
-    CK(cudaMemsetAsync(h->base + L.off_res, 0, res_scratch_bytes(L.P, L.NZ), h->stream));
+    count_hand_overs(h, em2_hand_overs((int)nsteps));
     CK(em2_resident_launch(fr, h->stream));
     return em2_adjoint_sweep_on_chip(h, A, s0, nsteps);
   }

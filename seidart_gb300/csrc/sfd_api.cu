@@ -22,7 +22,7 @@
 
 namespace sfd {
 
-__global__ void k_begin(Ctl* ctl, float* slots, int nslots, int step) {
+__global__ void k_begin(Ctl* ctl, float* slots, int nslots, int step, int hand_overs) {
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   for (int s = tid; s < nslots; s += gridDim.x * blockDim.x) slots[s] = 0.0f;
   if (tid == 0) {
@@ -31,8 +31,11 @@ __global__ void k_begin(Ctl* ctl, float* slots, int nslots, int step) {
     ctl->maxnorm = 0.0f;
     ctl->nan_seen = 0;
     ctl->err = 0;
+    ctl->seq += (unsigned)hand_overs;
   }
 }
+
+__global__ void k_count(Ctl* ctl, int hand_overs) { ctl->seq += (unsigned)hand_overs; }
 
 __global__ void k_advance(Ctl* ctl, int by) { ctl->base += by; }
 
@@ -58,10 +61,14 @@ using namespace sfd;
 
 namespace sfd {
 
-void begin_run(sfd_handle_s* h, int64_t step) {
+void begin_run(sfd_handle_s* h, int64_t step, int hand_overs) {
   const Layout& L = h->L;
   k_begin<<<std::min(1024, (L.nslots + 255) / 256 + 1), 256, 0, h->stream>>>(
-      (Ctl*)(h->base + L.off_ctl), (float*)(h->base + L.off_slots), L.nslots, (int)step);
+      (Ctl*)(h->base + L.off_ctl), (float*)(h->base + L.off_slots), L.nslots, (int)step, hand_overs);
+}
+
+void count_hand_overs(sfd_handle_s* h, int hand_overs) {
+  k_count<<<1, 1, 0, h->stream>>>((Ctl*)(h->base + h->L.off_ctl), hand_overs);
 }
 
 void reduce_norms(sfd_handle_s* h) {
@@ -268,6 +275,11 @@ void make_layout(const sfd_config& c, Layout* L) {
   if (single_pass(c) && !(c.flags & SFD_FLAG_STREAMING)) {
     L->off_res = o;  // edge arrays of on-chip runs
     o += align256(res_scratch_bytes(L->P, c.nz, res_edge_fields(c.kind)));
+  }
+  L->off_words = 0;
+  if (L->off_res && c.kind == SFD_ELECTROMAG2 && (size_t)L->P * c.nz <= kEm2MaxCells) {
+    L->off_words = o;  // hand-over words of on-chip runs
+    o += align256(em2_word_bytes(L->P, c.nz, c.npml));
   }
   L->total = o;
 }
@@ -532,36 +544,10 @@ bool resident_usable(sfd_handle* h) {
     h->res_state = 1;
     return true;
   }
-  // Plans are searched once per grid shape and device (the search takes
-  // tens of milliseconds; a survey creates one handle per shot).
-  // The forward kernel's plan (interior tiles with kResRows3 rows per
-  // thread) and the adjoint sweep's (kResRows everywhere).
-  struct PlanKey {
-    int nx, nz, npml, ctas, dev;
-    size_t smem;
-    bool rows3;
-  };
-  static std::mutex plan_mu;
-  static std::vector<std::pair<PlanKey, std::pair<bool, ResPlan>>> plans;
-  auto plan_for = [&](bool rows3, ResPlan* plan) {
-    const PlanKey key{h->cfg.nx, h->cfg.nz, h->cfg.npml, std::min(nsm, h->L.nslots), dev, (size_t)optin - static_smem,
-                      rows3};
-    {
-      std::lock_guard<std::mutex> lock(plan_mu);
-      for (const auto& e : plans)
-        if (e.first.nx == key.nx && e.first.nz == key.nz && e.first.npml == key.npml && e.first.ctas == key.ctas &&
-            e.first.dev == key.dev && e.first.smem == key.smem && e.first.rows3 == key.rows3) {
-          *plan = e.second.second;
-          return e.second.first;
-        }
-    }
-    const bool fits = em2_resident_plan(key.nx, key.nz, key.npml, key.ctas, key.smem, plan, rows3);
-    std::lock_guard<std::mutex> lock(plan_mu);
-    plans.push_back({key, {fits, *plan}});
-    return fits;
-  };
-  ResPlan plan;
-  if (!plan_for(true, &plan) || !plan_for(false, &h->res_plan_adj)) return false;
+  if (!h->L.off_words) return false;
+  Em2Plan plan;  // searched in tens of microseconds, not cached
+  if (!em2_resident_plan(h->cfg.nx, h->cfg.nz, h->cfg.npml, std::min(nsm, h->L.nslots), (size_t)optin - static_smem, &plan))
+    return false;
   int per_sm = 0;
   if (em2_resident_prepare(plan, &per_sm) != cudaSuccess || per_sm < 1) {
     cudaGetLastError();
@@ -570,6 +556,38 @@ bool resident_usable(sfd_handle* h) {
   h->res_plan = plan;
   h->res_state = 1;
   return true;
+}
+
+// The adjoint sweep's plans are searched once per grid shape and device (the
+// search takes tens of milliseconds).
+bool adjoint_plan(sfd_handle* h) {
+  int dev = 0, nsm = 0, optin = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  struct PlanKey {
+    int nx, nz, npml, ctas, dev;
+    size_t smem;
+  };
+  static std::mutex plan_mu;
+  static std::vector<std::pair<PlanKey, std::pair<bool, ResPlan>>> plans;
+  const PlanKey key{h->cfg.nx, h->cfg.nz, h->cfg.npml, std::min(nsm, h->L.nslots), dev, (size_t)optin - 8192};
+  {
+    std::lock_guard<std::mutex> lock(plan_mu);
+    for (const auto& e : plans)
+      if (e.first.nx == key.nx && e.first.nz == key.nz && e.first.npml == key.npml && e.first.ctas == key.ctas &&
+          e.first.dev == key.dev && e.first.smem == key.smem) {
+        h->res_plan_adj = e.second.second;
+        return e.second.first;
+      }
+  }
+  const bool fits = em2_adj_resident_plan(key.nx, key.nz, key.npml, key.ctas, key.smem, &h->res_plan_adj);
+  std::lock_guard<std::mutex> lock(plan_mu);
+  plans.push_back({key, {fits, h->res_plan_adj}});
+  return fits;
 }
 
 Em2Resident resident_args(const sfd_handle* h, int64_t nsteps) {
@@ -582,10 +600,7 @@ Em2Resident resident_args(const sfd_handle* h, int64_t nsteps) {
   r.X = b.X; r.Z = b.Z; r.dbH = b.dbH;
   r.io = b.io;
   r.plan = h->res_plan;
-  char* base = h->base + h->L.off_res;
-  r.r.erow = (uint2*)base;
-  r.r.NZp = res_nzp(h->cfg.nz);
-  r.r.ecol = r.r.erow + 4 * kResMaxTiles1D * (size_t)h->L.P;
+  r.words = (uint4*)(h->base + h->L.off_words);
   r.t0 = (int)h->step;
   r.nsteps = (int)nsteps;
   r.limit_ns = h->wait_ns;
@@ -1524,12 +1539,16 @@ int32_t sfd_run(sfd_handle* h, int64_t nsteps) {
   const Layout& L = h->L;
   Ctl* ctl = (Ctl*)(h->base + L.off_ctl);
   float* slots = (float*)(h->base + L.off_slots);
-  k_begin<<<std::min(1024, (L.nslots + 255) / 256 + 1), 256, 0, h->stream>>>(ctl, slots, L.nslots, (int)h->step);
-  if (resident_usable(h)) {  // the whole run in one launch, state on chip
-    // tags from an earlier run must not match: clear every edge word
-    CK(cudaMemsetAsync(h->base + L.off_res, 0, res_scratch_bytes(L.P, L.NZ, res_edge_fields(h->cfg.kind)), h->stream));
-    if (h->cfg.kind == SFD_SEISMIC2) CK(seis2_resident_launch(seis2_resident_args(h, nsteps), h->stream));
-    else CK(em2_resident_launch(resident_args(h, nsteps), h->stream));
+  const bool on_chip = resident_usable(h), em2 = h->cfg.kind == SFD_ELECTROMAG2;
+  begin_run(h, h->step, on_chip && em2 ? em2_hand_overs((int)nsteps) : 0);
+  if (on_chip) {  // the whole run in one launch, state on chip
+    if (em2) {
+      CK(em2_resident_launch(resident_args(h, nsteps), h->stream));
+    } else {
+      // tags from an earlier run must not match: clear every edge word
+      CK(cudaMemsetAsync(h->base + L.off_res, 0, res_scratch_bytes(L.P, L.NZ, res_edge_fields(h->cfg.kind)), h->stream));
+      CK(seis2_resident_launch(seis2_resident_args(h, nsteps), h->stream));
+    }
     k_reduce_slots<<<1, 1024, 0, h->stream>>>(ctl, slots, L.nslots);
     CK(cudaGetLastError());
     h->step += nsteps;
@@ -1626,9 +1645,7 @@ int32_t sfd_launch_half(sfd_handle* h, int32_t which, int32_t count) {
   if (which != 0 && which != 1) return fail(SFD_ERR_BAD_ARG, "which must be 0 or 1");
   if (count < 0) return fail(SFD_ERR_BAD_ARG, "count must be >= 0");
   if (!h->have_model || !h->have_cpml) return fail(SFD_ERR_STATE, "sfd_launch_half needs sfd_set_model and sfd_set_cpml");
-  const Layout& L = h->L;
-  k_begin<<<std::min(1024, (L.nslots + 255) / 256 + 1), 256, 0, h->stream>>>((Ctl*)(h->base + L.off_ctl),
-                                                                            (float*)(h->base + L.off_slots), L.nslots, 0);
+  begin_run(h, 0);
   for (int q = 0; q < count; ++q) {
     if (h->single) {
       launch_step(h, h->cur, 0, h->stream);  // the single-pass kernel is the whole step

@@ -25,7 +25,7 @@ struct Ctl {
   int base;       // global index of the step the next launch with rel = 0 computes
   int run_start;  // first step of the current sfd_run
   int err;       // a bounded device wait of the last run gave up
-  int pad1;
+  unsigned seq;   // tag of the last hand-over of on-chip runs up to and including the current one
   float maxnorm;  // largest field norm of the last run (after finalize)
   int nan_seen;
   int pad2, pad3;
@@ -128,7 +128,7 @@ __device__ __forceinline__ void gather_receivers(const int* __restrict__ rec, in
   }
 }
 
-__global__ void k_begin(Ctl* ctl, float* slots, int nslots, int step);
+__global__ void k_begin(Ctl* ctl, float* slots, int nslots, int step, int hand_overs);
 __global__ void k_advance(Ctl* ctl, int by);
 __global__ void k_reduce_slots(Ctl* ctl, const float* slots, int nslots);
 

@@ -56,6 +56,7 @@ const char* mem_axes(int kind);
 int ncoef(int kind);
 size_t align256(size_t x);
 bool cpml2d(const sfd_config& c);
+bool legacy_quirks(const sfd_config& c);
 // Whether a handle steps in the single-pass form (the others: two kernels per step).
 bool single_pass(const sfd_config& c);
 // Edge fields of an on-chip run (resident.h): electromag2 2, seismic2 6.
@@ -94,9 +95,9 @@ struct sfd_handle_s {
   sfd::Seis2Step s2s[2];
   sfd::Launch launch1;       // single-pass geometry
   int res_state = 0;    // on-chip runs: 0 not yet checked, 1 usable, -1 not usable
-  sfd::Em2Plan res_plan;     // electromag2
+  sfd::TilePlan res_plan;     // electromag2, seismic2
   sfd::ResPlan res_plan_adj;  // electromag2, the adjoint sweep's
-  sfd::Seis2ResPlan s2_plan;  // seismic2
+  sfd::Seis2ResPlan s2_plan;  // seismic2 with the legacy quirks
   int64_t step = 0;
   unsigned long long wait_ns = sfd::kDefaultWaitNs;  // longest wait of an on-chip run for a neighbouring tile
   bool stall_waits = false;                          // timeout test aid: waits expect tags no tile writes

@@ -45,12 +45,12 @@ struct ResPlan {
   size_t smem;  // dynamic shared memory of the largest tile
 };
 
-// Tiling of one electromag2 run: tile columns of about equal width, each cut
-// into its own bands (at most ntz).  tile[b] packs the owned cells, x0 | x1 <<
-// 16 and z0 | z1 << 16 (column bounds are multiples of 4 except NX), and
-// whether the frame holds strip or boundary cells (1) and x-strip ones (2).  A CTA has `warps` warps of
-// rb frame rows.
-struct Em2Plan {
+// Tiling of an on-chip run (tile_plan.h): tile columns of about equal width,
+// each cut into its own bands (at most ntz).  tile[b] packs the owned cells, x0
+// | x1 << 16 and z0 | z1 << 16 (column bounds are multiples of the cells a
+// lane holds, except NX), and whether the frame holds strip or boundary cells
+// (1) and x-strip ones (2).  A CTA has `warps` warps of rb frame rows.
+struct TilePlan {
   int ntiles, ntz, rb, warps;
   int4 tile[kResMaxTiles];
   size_t smem;  // dynamic shared memory of the largest tile
@@ -63,6 +63,19 @@ struct Em2Plan {
 inline size_t em2_word_bytes(int P, int NZ, int W) {
   return 2 * sizeof(uint4) * ((size_t)NZ * P + 2 * (size_t)W * P + (size_t)NZ * 2 * W);
 }
+// The seismic2 runs' tiles (resident_s2.cu): two cells a lane; a step moves
+// information by two cells, so kS2Halo cells of halo last kS2Halo / 2 steps.
+constexpr int kS2Halo = 4;
+constexpr int kS2Steps = kS2Halo / 2;
+constexpr int kS2MaxRows = 3;
+// Their hand-over words, two copies, each: {vx, vz, sxx, tag} and {szz, sxz,
+// -, tag} by cell [NZ][2][P], the z strips' six memory variables in two words
+// a cell [2W][2][P] and the x strips' [NZ][2][2W].
+inline size_t s2_word_bytes(int P, int NZ, int W) {
+  return 2 * sizeof(uint4) * 2 * ((size_t)NZ * P + 2 * (size_t)W * P + (size_t)NZ * 2 * W);
+}
+constexpr size_t kS2MaxCells = (size_t)kResMaxTiles * 60 * kS2MaxRows * 16;
+__host__ __device__ inline int s2_hand_overs(int nsteps) { return nsteps <= kS2Steps ? 1 : (nsteps - 1) / kS2Steps; }
 // Largest grid (cells of pitch) an electromag2 run can hold on chip; larger
 // ones get no hand-over words.
 constexpr size_t kEm2MaxCells = (size_t)kResMaxTiles * 124 * kEm2MaxRows * kEm2MaxWarps;
@@ -127,7 +140,7 @@ struct Em2Resident {
   AxisTab X, Z;
   float dbH;
   IoArgs io;
-  Em2Plan plan;
+  TilePlan plan;
   uint4* words;
   int t0, nsteps;
   unsigned long long limit_ns;  // longest wait for a neighbour before the run is abandoned
@@ -167,7 +180,7 @@ struct Em2AdjResident {
   unsigned long long limit_ns;
 };
 
-// On-chip seismic2 run: a uniform ntx x ntz grid of tiles, tile (c, r)
+// On-chip seismic2 run with the legacy quirks: a uniform ntx x ntz grid of tiles, tile (c, r)
 // covering columns [xb[c], xb[c+1]) and rows [zb[r], zb[r+1]).
 struct Seis2ResPlan {
   int ntx, ntz;
@@ -194,8 +207,10 @@ struct Seis2Resident {
   const float* q3;
   AxisTab X, Z;
   IoArgs io;
-  Seis2ResPlan plan;
-  ResScratch r;  // six edge fields
+  TilePlan tiles;     // corrected physics
+  uint4* words;
+  Seis2ResPlan plan;  // legacy quirks: its tiles and six edge fields
+  ResScratch r;
   int t0, nsteps;
   unsigned long long limit_ns;
   unsigned tag_bias;  // added to every awaited edge tag; 0 except in the timeout test aid
@@ -203,18 +218,22 @@ struct Seis2Resident {
 };
 
 // Tiling of an NX x NZ seismic2 grid for `max_ctas` CTAs of at most
-// `max_smem` bytes; false when the grid does not fit on chip.
-bool seis2_resident_plan(int NX, int NZ, int max_ctas, size_t max_smem, Seis2ResPlan* out);
-cudaError_t seis2_resident_prepare(const Seis2ResPlan& plan, int* ctas_per_sm);
+// `max_smem` bytes; false when the grid does not fit on chip.  seis2_legacy_*:
+// the kernel that runs the legacy quirks (resident_s2_legacy.cu).
+bool seis2_resident_plan(int NX, int NZ, int npml, int max_ctas, size_t max_smem, TilePlan* out);
+cudaError_t seis2_resident_prepare(const TilePlan& plan, int* ctas_per_sm);
 cudaError_t seis2_resident_launch(const Seis2Resident& a, cudaStream_t s);
+bool seis2_legacy_plan(int NX, int NZ, int max_ctas, size_t max_smem, Seis2ResPlan* out);
+cudaError_t seis2_legacy_prepare(const Seis2ResPlan& plan, int* ctas_per_sm);
+cudaError_t seis2_legacy_launch(const Seis2Resident& a, cudaStream_t s);
 
 // Pick the tiling of an NX x NZ electromag2 grid with npml-cell strips for
 // `max_ctas` CTAs of at most `max_smem` bytes of shared memory.  Returns
 // false when the grid does not fit on chip.
-bool em2_resident_plan(int NX, int NZ, int npml, int max_ctas, size_t max_smem, Em2Plan* out);
+bool em2_resident_plan(int NX, int NZ, int npml, int max_ctas, size_t max_smem, TilePlan* out);
 // Set the kernels' shared-memory limit (once per device) and return how many
 // CTAs of the plan fit on one SM.
-cudaError_t em2_resident_prepare(const Em2Plan& plan, int* ctas_per_sm);
+cudaError_t em2_resident_prepare(const TilePlan& plan, int* ctas_per_sm);
 cudaError_t em2_resident_launch(const Em2Resident& a, cudaStream_t s);
 
 // The same for the adjoint sweep's tiles.

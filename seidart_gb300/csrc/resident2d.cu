@@ -1,7 +1,7 @@
 // SM-resident electromag2 run: every time step of an sfd_run in one
 // cooperative launch, with the whole state on chip.
 //
-// The grid is cut into tiles (Em2Plan), one CTA each for the whole run.  A
+// The grid is cut into tiles (TilePlan), one CTA each for the whole run.  A
 // tile is the frame of em2_tile.cuh: RB rows of 128 columns a warp, the
 // fields in registers, coefficients and CPML memory variables in shared
 // memory.  Every kTileHalo steps a tile writes the owned cells its
@@ -33,9 +33,9 @@
 // states of the plain run.
 #include <algorithm>
 #include <type_traits>
-#include <vector>
 
 #include "em2_tile.cuh"
+#include "tile_plan.h"
 
 namespace sfd {
 
@@ -759,28 +759,6 @@ const void* em2_kernel(int rb, int mode) {
 #define SFD_EM2_MIN_COST 16.0
 #endif
 
-struct Frame {
-  int rows, own, zlo, zhi, xlanes;  // rows, owned ones, those of the low and the high z strip, lanes with x-strip cells
-  int zhi0;                    // first row of the high z strip
-  bool edge;
-};
-
-Frame em2_frame(int NX, int NZ, int W, int ox0, int ox1, int oz0, int oz1) {
-  const int bx = ox0 > 0 ? ox0 - kTileHalo : 0, bz = std::max(oz0 - kTileHalo, 0);
-  const int xend = std::min(NX, ox1 + kTileHalo), kend = std::min(NZ, oz1 + kTileHalo);
-  Frame f;
-  f.rows = kend - bz;
-  f.own = oz1 - oz0;
-  f.zlo = std::max(std::min(W, kend) - bz, 0);
-  f.zhi0 = std::max(NZ - W, bz) - bz;
-  f.zhi = std::max(kend - std::max(NZ - W, bz), 0);
-  const int xlo = std::max((std::min(W, xend) - bx + 3) / 4, 0), xh0 = std::max((NX - W - bx) / 4, xlo);
-  f.xlanes = xlo + std::max((xend - bx + 3) / 4 - xh0, 0);
-  const int lo = std::max(W, 1);
-  f.edge = bx < lo || xend > NX - std::max(W, 2) || bz < lo || kend > NZ - std::max(W, 2);
-  return f;
-}
-
 // Shared memory of a frame with rb rows a warp, as em2_run_tile lays it out.
 size_t em2_tile_smem(const Frame& f, int rb) {
   const size_t R = (size_t)(f.rows + rb - 1) / rb * rb;
@@ -797,76 +775,12 @@ size_t em2_tile_smem(const Frame& f, int rb) {
 
 }  // namespace
 
-bool em2_resident_plan(int NX, int NZ, int npml, int max_ctas, size_t max_smem, Em2Plan* out) {
-  const int W = npml;
-  max_ctas = std::min(max_ctas, kResMaxTiles);
-  // tile columns: as few as there can be, of about equal width
-  const int ng = (NX + 3) / 4, inner = (kCols - 2 * kTileHalo) / 4;
-  const int ntx = NX <= kCols ? 1 : std::max(2, (ng - 2 + inner - 1) / inner);
-  std::vector<int> xb(ntx + 1);
-  for (int c = 0; c <= ntx; ++c)
-    xb[c] = ng <= inner * ntx || ntx == 1 ? (int)((long)c * ng / ntx) : c == 0 ? 0 : c == ntx ? ng : inner * c + 1;
-  for (int c = 0; c <= ntx; ++c) xb[c] = std::min(NX, 4 * xb[c]);
-  const int max_rows = kEm2MaxRows * kEm2MaxWarps;
-  // the bands of column c at cost C a tile, greedily from the top; false if a row alone is too much
-  auto bands = [&](int c, double C, std::vector<int>* cuts) {
-    int n = 0, z = 0;
-    if (cuts) cuts->assign(1, 0);
-    while (z < NZ) {
-      int z1 = z;
-      while (z1 < NZ) {
-        const Frame f = em2_frame(NX, NZ, W, xb[c], xb[c + 1], z, z1 + 1);
-        const double cost = (f.rows + SFD_EM2_ZROW_COST * (f.zlo + f.zhi)) * (f.xlanes ? 1.0 + SFD_EM2_XCOL_COST : 1.0);
-        if (cost > C || f.rows > max_rows || em2_tile_smem(f, kEm2MaxRows) > max_smem) break;
-        ++z1;
-      }
-      if (z1 == z) return max_ctas + 1;
-      // a last band of a few rows: no thinner than its neighbours' halo
-      if (NZ - z1 > 0 && NZ - z1 < kTileHalo) z1 = std::max(z + 1, NZ - kTileHalo);
-      z = z1;
-      ++n;
-      if (cuts) cuts->push_back(z);
-      if (n > max_ctas) break;
-    }
-    return n;
-  };
-  auto tiles_at = [&](double C) {
-    int total = 0;
-    for (int c = 0; c < ntx && total <= max_ctas; ++c) total += bands(c, C, nullptr);
-    return total;
-  };
-  double lo = SFD_EM2_MIN_COST - 0.5, hi = 2.0 * max_rows;
-  if (tiles_at(hi) > max_ctas) return false;
-  if (tiles_at(lo) <= max_ctas) hi = lo;
-  for (int it = 0; it < 24 && hi - lo > 0.25; ++it) {
-    const double mid = 0.5 * (lo + hi);
-    (tiles_at(mid) <= max_ctas ? hi : lo) = mid;
-  }
-  out->ntiles = out->ntz = 0;
-  int rows = 0;
-  std::vector<int> cuts;
-  for (int c = 0; c < ntx; ++c) {
-    bands(c, hi, &cuts);
-    out->ntz = std::max(out->ntz, (int)cuts.size() - 1);
-    for (size_t q = 0; q + 1 < cuts.size(); ++q) {
-      const Frame f = em2_frame(NX, NZ, W, xb[c], xb[c + 1], cuts[q], cuts[q + 1]);
-      rows = std::max(rows, f.rows);
-      out->tile[out->ntiles++] = make_int4(xb[c] | (xb[c + 1] << 16), cuts[q] | (cuts[q + 1] << 16), f.edge ? (f.xlanes ? 2 : 1) : 0, 0);
-    }
-  }
-  out->rb = 1;
-  while (rows > out->rb * kEm2MaxWarps) ++out->rb;
-  out->warps = (rows + out->rb - 1) / out->rb;
-  out->smem = 0;
-  for (int b = 0; b < out->ntiles; ++b) {
-    const int4 t = out->tile[b];
-    out->smem = std::max(out->smem, em2_tile_smem(em2_frame(NX, NZ, W, t.x & 0xffff, t.x >> 16, t.y & 0xffff, t.y >> 16),
-                                                  out->rb));
-  }
-  return out->smem <= max_smem;
+bool em2_resident_plan(int NX, int NZ, int npml, int max_ctas, size_t max_smem, TilePlan* out) {
+  const TileRules rules{4, kTileHalo, kEm2MaxRows, kEm2MaxWarps, SFD_EM2_ZROW_COST, SFD_EM2_XCOL_COST, SFD_EM2_MIN_COST};
+  return plan_tiles(rules, NX, NZ, npml, max_ctas, max_smem, em2_tile_smem, out);
 }
 
-cudaError_t em2_resident_prepare(const Em2Plan& plan, int* ctas_per_sm) {
+cudaError_t em2_resident_prepare(const TilePlan& plan, int* ctas_per_sm) {
   int n = 1 << 30;
   for (int mode = 0; mode < 3; ++mode) {
     const void* fn = em2_kernel(plan.rb, mode);

@@ -1,579 +1,833 @@
-// SM-resident seismic2 run: every time step of an sfd_run in one cooperative
-// launch, with the whole state on chip.
+// SM-resident seismic2 run (corrected physics): every time step of an sfd_run
+// in one cooperative launch, with the whole state on chip.
 //
-// The grid is cut into a uniform ntx x ntz grid of tiles (Seis2ResPlan), one
-// CTA per tile for the whole run.  A tile keeps, in shared memory, its five
-// fields with a one-cell halo ring, its twelve coefficient planes and its
-// twelve CPML memory variables (eight with the legacy quirks, where the two
-// stress loops share four).  The per-cell arithmetic is that of the
-// single-pass tile (fused2d.cuh: seis2_stress_cell and the per-cell velocity
-// code), i.e. the loops of legacy/fortran/seismicfdtd.f95:247-379, so the
-// streaming and on-chip forms give the same fields.
+// The tiles are those of the electromag2 run (em2_tile.cuh, resident2d.cu) for
+// the velocity-stress step: a warp holds RB whole rows of 64 columns, two cells
+// a lane, the five fields in registers; the twelve coefficients lie in
+// registers for RB = 1, else in shared memory, the CPML memory variables of
+// strip cells in shared memory.  A half-step needs its neighbours along x from
+// the next lanes (six shuffles a row and step) and along z from the next warps
+// (vx, vz of a warp's first and last row, szz of its first, sxz of its last
+// row through shared memory).  A step moves information by two cells -- the
+// stresses read velocities one cell away, the velocities stresses one cell away
+// -- so a halo of kS2Halo cells lasts kS2Steps steps; then the tiles hand over
+// {vx, vz, sxx, tag} and {szz, sxz, -, tag} of every halo cell, and the strips'
+// memory variables, through L2 as the electromag2 run does.
 //
-// A step is two half-steps, each followed by a halo exchange with the four
-// neighbouring tiles through tagged 8-byte edge words in global memory (L2),
-// as in the electromag2 on-chip run (resident2d.cu):
-//   stresses (:247-312) need vx, vz one cell left, right, above and below;
-//   velocities (:317-357) need sxx on the left, sxz above and on the right,
-//   szz below.
-// The cell warps compute a tile's perimeter cells first and write their edge
-// values as soon as they are computed (row edges indexed by tile row and
-// global x, column edges by tile column and global z, tag = one more than the
-// reading step, two copies by the parity of the reading step).  Meanwhile
-// four exchange warps, one per neighbour, poll the neighbours' words of the
-// same half-step until they carry the expected tag and copy them into the
-// halo ring, so the exchange overlaps the interior cells and a step needs
-// two block barriers.  A poll gives up after limit_ns (%globaltimer) or when
-// another tile has given up, records the failure in the control block, and
-// the CTA leaves the run; the host reports SFD_ERR_TIMEOUT.  The launch is
-// cooperative, so all tiles are co-resident and a correct run never reaches
-// the limit.
+// The Fortran's loop bounds (seismicfdtd.f95:247-357) are coefficient values:
+// sfd_set_model leaves the stiffness averages zero outside their loop, and
+// dt/rho of the outermost cells, where the velocities are Dirichlet planes, is
+// taken as zero.  A memory variable outside its loop is left to run in shared
+// memory -- it is only ever multiplied by such a zero -- and is not stored.
+//
+// What bounds it: as there, the chain of a step and the hand-over every
+// kS2Steps steps.  On 440 x 240 cells a step takes 2.32 us (3.4 us in the form
+// before it, which exchanged one-cell edges twice a step and read every operand
+// from shared memory), on 120 x 90 cells 1.85 us.  Halos of 6 and 8 cells (3
+// and 4 steps a hand-over) run 2.47 and 2.29 us: what they save in hand-overs
+// they compute twice.  Frames of one row a warp (21 warps) run 2.84 us.
+//
+// Every product and sum names its rounding, so that a cell gets the same bits
+// from whichever tile computes it and a run in pieces, or recomputed for the
+// adjoint, gives the states of the plain run.
 #include <algorithm>
+#include <type_traits>
 
-#include "resident_common.cuh"
+#include "em2_tile.cuh"
+#include "tile_plan.h"
 
 namespace sfd {
 
 using namespace res;
+using tile2::ld_word;
+using tile2::max_nan;
+using tile2::norm_of_sq;
+using tile2::norm_sq;
+using tile2::poll_again;
+using tile2::st_word;
 
 namespace {
 
-constexpr int kS2ExchangeWarps = 4;
-constexpr int kS2CellThreads = 256;
-constexpr int kS2Threads = 32 * kS2ExchangeWarps + kS2CellThreads;
-constexpr int kS2MaxTile = 128;  // tile width and height: two fields of one side fit one warp's poll
+constexpr int kSC = 64;       // frame columns: 32 lanes x 2 cells
+constexpr int kS2Warps = 16;  // most warps of a CTA
+constexpr int kS2Keep = 1;    // up to this many rows a warp the coefficients stay in registers
+constexpr int kS2Batch = 3;   // words a thread has in flight in a hand-over
+// places in s2_smem (floats): x tables ik ad b ikh adh bh, each warp's first
+// vx, first vz, last vx, last vz, each warp's first szz, last sxz, row tables
+// [48][8] ik ikh - - b ad bh adh, coefficients [R][12][64]
+constexpr int kSV = 6 * kSC, kSS = kSV + kS2Warps * 4 * kSC, kSRT = kSS + kS2Warps * 2 * kSC,
+              kSCo = kSRT + 8 * kS2MaxRows * kS2Warps;
 
-// Fields with their halo ring, coefficients, memory variables and the axis
-// tables of the tile's columns and rows (floats), then the cell order
-// (16-bit (row << 7) | column per cell).
-size_t s2_smem(int TW, int TZ) {
-  return sizeof(float) * (5 * (size_t)(TZ + 2) * (TW + 2) + 24 * (size_t)TZ * TW + 6 * (size_t)TW + 7 * (size_t)TZ) +
-         2 * (((size_t)TZ * TW + 1) & ~(size_t)1);
+extern __shared__ __align__(16) float s2_smem[];
+
+__device__ __forceinline__ float& el(float2& v, int e) { return (&v.x)[e]; }
+__device__ __forceinline__ float el(const float2& v, int e) { return (&v.x)[e]; }
+__device__ __forceinline__ float2 lds(int o) { return *reinterpret_cast<const float2*>(s2_smem + o); }
+__device__ __forceinline__ void sts(int o, float2 v) { *reinterpret_cast<float2*>(s2_smem + o) = v; }
+
+// Place of cell i's word w of row k among the hand-over words (a warp's store
+// of one cell and word of every lane writes 512 consecutive bytes).
+__device__ __forceinline__ int s2_word(int k, int w, int i, int P) {
+  return ((2 * k + w) * 2 + (i & 1)) * (P >> 1) + (i >> 1);
 }
 
-// One warp: copy n words of src0 into dst0[q * st0] and, when src1 is given,
-// n words of src1 into dst1[q * st1], each once its tag reads `tag`.  Each
-// lane issues the loads of all its pending words before testing any.  False
-// (on every lane) if the wait gave up.
-__device__ __noinline__ bool fetch2(const uint2* src0, float* dst0, int st0, const uint2* src1, float* dst1, int st1,
-                                    int n, unsigned tag, Ctl* ctl, unsigned long long limit_ns) {
-  const int lane = threadIdx.x & 31;
-  const int total = (src1 ? 2 : 1) * n;
-  unsigned pending = 0;
-#pragma unroll
-  for (int k = 0; k < kResFetchPerLane; ++k)
-    if (lane + 32 * k < total) pending |= 1u << k;
-  bool ok = true;
-  unsigned long long t0 = 0;
-  uint2 v[kResFetchPerLane];
-  for (int it = 1; pending; ++it) {
-#pragma unroll
-    for (int k = 0; k < kResFetchPerLane; ++k) {
-      const int q = lane + 32 * k;
-      if (pending & (1u << k)) v[k] = ld_vol2(q < n ? src0 + q : src1 + (q - n));
-    }
-#pragma unroll
-    for (int k = 0; k < kResFetchPerLane; ++k) {
-      const int q = lane + 32 * k;
-      if ((pending & (1u << k)) && v[k].y == tag) {
-        if (q < n) dst0[q * st0] = __uint_as_float(v[k].x);
-        else dst1[(q - n) * st1] = __uint_as_float(v[k].x);
-        pending &= ~(1u << k);
-      }
-    }
-    if (pending && (it & 7) == 0 && !keep_polling(ctl, limit_ns, t0)) {
-      ok = false;
-      break;
-    }
-  }
-  return __all_sync(0xffffffffu, ok);
+// Most entries of the lists of a hand-over: of a tile with hrows halo rows, hown
+// owned rows, zrows frame rows in a z strip, xlanes lanes with x-strip cells
+// (two words a cell, fields and strips alike).
+__host__ __device__ constexpr int s2_get_entries(int hrows, int hown, int zrows, int xlanes) {
+  return 2 * ((hrows + (hrows < zrows ? hrows : zrows)) * kSC + 2 * kS2Halo * (hown + (hown < zrows ? hown : zrows)) +
+              2 * xlanes * hrows + (xlanes ? 2 * kS2Halo * hown : 0));
+}
+__host__ __device__ constexpr int s2_pub_entries(int hown, int zrows, int xlanes) {
+  return 2 * ((2 * kS2Halo < zrows ? 2 * kS2Halo : zrows) * kSC + 2 * kS2Halo * (hown < zrows ? hown : zrows) +
+              2 * xlanes * 2 * kS2Halo + (xlanes ? 2 * kS2Halo * hown : 0));
 }
 
-// Edge fields: rows (indexed by tile row and global x) and columns (by tile
-// column and global z).
-enum : int {
-  kEVxFirst = 0,  // vx, vz first row / column: read by the tile above / left
-  kEVzFirst = 1,
-  kEVxLast = 2,   // vx, vz last row / column: read by the tile below / right
-  kEVzLast = 3,
-  kESFirst = 4,   // szz first row (tile above), sxz first column (tile left)
-  kESLast = 5     // sxz last row (tile below), sxx last column (tile right)
+// A tile's geometry and the places of its arrays, in shared memory (as Em2Tile).
+struct S2Tile {
+  int ox0, ox1, oz0, oz1, bx, bz, xend, kend;
+  int wlo, wh0, xlo, xh0, nxl;  // warps and lanes with strip cells, as in Em2Tile
+  int R, zn, hS;                // frame rows in whole warps, those of a z strip, floats of a field of the halo
+  unsigned tag;
+  int nrec, nmine, abort;
+  int oZ, oX, oH, oGet, oPub, nget, npub;
+  int rec[2 * kResMaxLocalRec], mine[kResMaxLocalRec];
 };
 
-// DUMP: a recompute for the adjoint -- every step's state written to its
-// slot, the loaded state not written back.
-template <bool DUMP>
-__global__ void __launch_bounds__(kS2Threads, 1) seis2_resident_kernel(const __grid_constant__ Seis2Resident a) {
-  extern __shared__ __align__(16) float smem[];
-  __shared__ int s_abort, s_nrec;
-  __shared__ int s_rec[2 * kResMaxLocalRec];  // (receiver, halo-frame cell) pairs
+// Memory variable q of the z strips' six and of the x strips' six, in
+// sfd_num_memory's order, and whether cell (i, k) lies in the loop that
+// advances it: 0, 1 the normal stresses', 2, 3 the shear stress's, 4, 5 the
+// velocities'.
+__device__ __forceinline__ constexpr int z_index(int q) { return q == 0 ? 1 : q == 1 ? 2 : q == 2 ? 9 : q == 3 ? 10 : q == 4 ? 5 : 7; }
+__device__ __forceinline__ constexpr int x_index(int q) { return q == 0 ? 0 : q == 1 ? 3 : q == 2 ? 8 : q == 3 ? 11 : q == 4 ? 4 : 6; }
+__device__ __forceinline__ bool in_loop(bool zstrip, int q, int i, int k, int NX, int NZ) {
+  if (q < 2) return k >= 1 && i <= NX - 2;
+  if (q < 4) return k <= NZ - 2 && i >= 1;
+  return (q == 4) == zstrip ? k <= NZ - 2 && i <= NX - 2 : k >= 1 && i >= 1;  // szz_z, sxz_x: vz; sxz_z, sxx_x: vx
+}
+
+template <int RB, bool DUMP, bool EDGE, bool XS>
+__device__ __forceinline__ void s2_run_tile(const Seis2Resident& a, S2Tile& G) {
+  constexpr bool KEEP = RB <= kS2Keep;
+  constexpr int kRow = 12 * kSC;
   const int NX = a.NX, NZ = a.NZ, P = a.P, W = a.W;
-  const int ntx = a.plan.ntx, ntz = a.plan.ntz;
-  const int bx = blockIdx.x % ntx, bz = blockIdx.x / ntx;
-  const int x0 = a.plan.xb[bx], x1 = a.plan.xb[bx + 1], z0 = a.plan.zb[bz], z1 = a.plan.zb[bz + 1];
-  const int tw = x1 - x0, tz = z1 - z0, SW = tw + 2, FS = (tz + 2) * SW, CS = tw * tz;
-  const bool up = bz > 0, down = bz < ntz - 1, left = bx > 0, right = bx < ntx - 1;
-  float* F = smem;         // vx vz sxx szz sxz, (tz + 2) x (tw + 2) with the halo ring
-  float* C = F + 5 * FS;   // A11 A13 A15 A33 A35 B15 B35 B55 dtrx dtrz gxp gzp, tz x tw
-  // m_vxx m_vzz m_vxz m_vzx m_sxx_x m_szz_z m_sxz_x m_sxz_z, then the sigmaxz
-  // loop's own m2_vxx m2_vzz m2_vxz m2_vzx (corrected physics), tz x tw each
-  float* M = C + 12 * CS;
-  float* XT = M + 12 * CS;  // x tables at the tile's columns: ik ad b ikh adh bh, tw each
-  float* ZT = XT + 6 * tw;  // z tables at the tile's rows, then q3, tz each
-  unsigned short* CELL = reinterpret_cast<unsigned short*>(ZT + 7 * tz);  // cell order, see cell_at
-  float* VX = F;
-  float* VZ = F + FS;
-  float* SXX = F + 2 * FS;
-  float* SZZ = F + 3 * FS;
-  float* SXZ = F + 4 * FS;
-  const int tid = threadIdx.x, warp = tid >> 5;
-  auto fi = [&](int lr, int lc) { return (lr + 1) * SW + lc + 1; };
-  Ctl* ctl = a.io.ctl;
-  const int NZp = a.r.NZp;
-  auto erow = [&](int par, int f, int b) { return a.r.erow + (size_t)((par * 6 + f) * kResMaxTiles1D + b) * P; };
-  auto ecol = [&](int par, int f, int b) { return a.r.ecol + (size_t)((par * 6 + f) * kResMaxTiles1D + b) * NZp; };
-
-  // ---- load the tile: fields, the velocities of the halo ring (the
-  // stresses of the ring are exchanged every step), coefficients, memory
-  for (int q = tid; q < 5 * FS + 24 * CS; q += kS2Threads) smem[q] = 0.0f;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const float2 zero2 = make_float2(0.f, 0.f);
+  Ctl* const ctl = a.io.ctl;
+  const int4 te = a.tiles.tile[blockIdx.x];
+  const bool up = (te.y & 0xffff) > 0, down = (te.y >> 16) < NZ, left = (te.x & 0xffff) > 0, right = (te.x >> 16) < NX;
+  const bool neighbours = up || down || left || right;
+  float* const memory[12] = {a.m_vxx, a.m_vzz, a.m_vxz, a.m_vzx, a.m_sxx_x, a.m_szz_z,
+                             a.m_sxz_x, a.m_sxz_z, a.m2_vxx, a.m2_vzz, a.m2_vxz, a.m2_vzx};
   if (tid == 0) {
-    s_nrec = 0;
-    s_abort = 0;
+    G.ox0 = te.x & 0xffff; G.ox1 = te.x >> 16; G.oz0 = te.y & 0xffff; G.oz1 = te.y >> 16;
+    G.bx = left ? G.ox0 - kS2Halo : 0;
+    G.bz = max(G.oz0 - kS2Halo, 0);
+    G.xend = min(NX, G.ox1 + kS2Halo);
+    G.kend = min(NZ, G.oz1 + kS2Halo);
+    G.R = (G.kend - G.bz + RB - 1) / RB * RB;
+    G.zn = max(min(W, G.kend) - G.bz, 0) + max(G.kend - max(NZ - W, G.bz), 0);
+    G.wlo = (max(min(W, G.kend) - G.bz, 0) + RB - 1) / RB;
+    G.wh0 = max((max(NZ - W, G.bz) - G.bz) / RB, G.wlo);
+    G.xlo = max((min(W, G.xend) - G.bx + 1) / 2, 0);
+    G.xh0 = max((NX - W - G.bx) / 2, G.xlo);
+    G.nxl = G.xlo + max((G.xend - G.bx + 1) / 2 - G.xh0, 0);
+    G.oZ = kSCo + (KEEP ? 0 : kRow * G.R);
+    G.oX = G.oZ + (EDGE ? 6 * kSC * RB * (G.wlo + max(G.R / RB - G.wh0, 0)) : 0);
+    G.oH = G.oX + (EDGE ? 12 * G.R * G.nxl : 0);
+    const int hown = G.oz1 - G.oz0, hrows = G.oz0 - G.bz + G.kend - G.oz1;
+    G.hS = hrows * kSC + 2 * kS2Halo * hown;
+    G.oGet = (G.oH + 6 * G.hS + 1) & ~1;
+    G.oPub = G.oGet + 2 * s2_get_entries(hrows, hown, EDGE ? G.zn : 0, EDGE ? G.nxl : 0);
+    G.nrec = G.nmine = G.nget = G.npub = G.abort = 0;
+    G.tag = *(volatile unsigned*)&ctl->seq - (unsigned)s2_hand_overs(a.nsteps);  // k_begin counted this run's on
   }
+  for (int q = tid; q < kS2Warps * 6 * kSC; q += blockDim.x) s2_smem[kSV + q] = 0.0f;  // rows past the frame are read as zero
   __syncthreads();
-  for (int q = tid; q < FS; q += kS2Threads) {
-    const int lr = q / SW - 1, lc = q % SW - 1, k = z0 + lr, i = x0 + lc;
-    const bool rin = lr >= 0 && lr < tz, cin = lc >= 0 && lc < tw;
-    if (k < 0 || k >= NZ || i < 0 || i >= NX || (!rin && !cin)) continue;
-    const size_t g = (size_t)k * P + i;
-    VX[q] = a.vx[g];
-    VZ[q] = a.vz[g];
-    if (rin && cin) {
-      SXX[q] = a.sxx[g];
-      SZZ[q] = a.szz[g];
-      SXZ[q] = a.sxz[g];
-    }
-  }
-  for (int q = tid; q < CS; q += kS2Threads) {
-    const int lr = q / tw, lc = q - lr * tw, k = z0 + lr, i = x0 + lc;
-    const size_t g = (size_t)k * P + i;
-#pragma unroll
-    for (int c = 0; c < 12; ++c) C[c * CS + q] = a.coef[c][g];
-    if (in_strip(i, NX, W)) {
-      const size_t mx = (size_t)k * (2 * W) + strip_idx(i, NX, W);
-      M[0 * CS + q] = a.m_vxx[mx];
-      M[3 * CS + q] = a.m_vzx[mx];
-      M[4 * CS + q] = a.m_sxx_x[mx];
-      M[6 * CS + q] = a.m_sxz_x[mx];
-      if (!a.legacy) {
-        M[8 * CS + q] = a.m2_vxx[mx];
-        M[11 * CS + q] = a.m2_vzx[mx];
-      }
-    }
-    if (in_strip(k, NZ, W)) {
-      const size_t mz = (size_t)strip_idx(k, NZ, W) * P + i;
-      M[1 * CS + q] = a.m_vzz[mz];
-      M[2 * CS + q] = a.m_vxz[mz];
-      M[5 * CS + q] = a.m_szz_z[mz];
-      M[7 * CS + q] = a.m_sxz_z[mz];
-      if (!a.legacy) {
-        M[9 * CS + q] = a.m2_vzz[mz];
-        M[10 * CS + q] = a.m2_vxz[mz];
-      }
-    }
-  }
-  {
-    const float* xs[6] = {a.X.ik, a.X.ad, a.X.b, a.X.ikh, a.X.adh, a.X.bh};
-    const float* zs[7] = {a.Z.ik, a.Z.ad, a.Z.b, a.Z.ikh, a.Z.adh, a.Z.bh, a.q3};
-    for (int q = tid; q < 6 * tw; q += kS2Threads) XT[q] = xs[q / tw][x0 + q % tw];
-    for (int q = tid; q < 7 * tz; q += kS2Threads) ZT[q] = zs[q / tz][z0 + q % tz];
-  }
-  for (int q = tid; q < a.io.nrec; q += kS2Threads) {  // receivers of this tile
-    const int i = a.io.rec[3 * q], k = a.io.rec[3 * q + 2];
-    if (i >= x0 && i < x1 && k >= z0 && k < z1) {
-      const int pos = atomicAdd(&s_nrec, 1);
-      if (pos < kResMaxLocalRec) {
-        s_rec[2 * pos] = q;
-        s_rec[2 * pos + 1] = fi(k - z0, i - x0);
-      }
-    }
-  }
-  __syncthreads();
-  const int nloc = s_nrec;
-  const int si = a.io.si, sk = a.io.sk;
+  const int nr = min(max(G.kend - G.bz - warp * RB, 0), RB);  // frame rows of this warp
+  const int oC = kSCo + warp * RB * kRow + 2 * lane, oRT = kSRT + 8 * warp * RB;
+  const bool xsl = XS && nr > 0 && G.bx + 2 * lane < G.xend && (lane < G.xlo || lane >= G.xh0);
+  const bool zw = EDGE && nr > 0 && (warp < G.wlo || warp >= G.wh0);
+  const int oZ = G.oZ + 6 * kSC * RB * (warp < G.wlo ? warp : warp - G.wh0 + G.wlo) + 2 * lane;  // + (6 j + q) kSC
+  const int sX = 2 * G.nxl;
+  const int oX = G.oX + 6 * sX * RB * warp + 2 * (lane < G.xlo ? lane : lane - G.xh0 + G.xlo);  // + (6 j + q) sX
 
-  // Cell n of this tile in perimeter-first order: the first and last rows,
-  // then the first and last columns, then the interior row by row.
-  // Tabulated once (CELL) so the steps do no division.
-  auto cell_order = [&](int n, int& lr, int& lc) {
-    if (tz <= 2 || tw <= 2) {
-      lr = n / tw;
-      lc = n - lr * tw;
-    } else if (n < 2 * tw) {
-      lr = n < tw ? 0 : tz - 1;
-      lc = n < tw ? n : n - tw;
-    } else if (n < 2 * tw + 2 * (tz - 2)) {
-      const int m = n - 2 * tw;
-      lr = 1 + (m < tz - 2 ? m : m - (tz - 2));
-      lc = m < tz - 2 ? 0 : tw - 1;
-    } else {
-      const int m = n - 2 * tw - 2 * (tz - 2);
-      lr = 1 + m / (tw - 2);
-      lc = 1 + m % (tw - 2);
+  // ---- load the frame
+  float2 vx[RB], vz[RB], sxx[RB], szz[RB], sxz[RB], keep[KEEP ? RB : 1][12];
+  unsigned own = 0, plane = 0;  // owned rows of this lane; cells (bit 2 * row + element) on a Dirichlet plane
+  int src = -1;                 // 2 * row + element of the source cell
+  {
+    const int i0 = G.bx + 2 * lane, kb = G.bz + warp * RB;
+    const bool lact = i0 < G.xend, lown = i0 >= G.ox0 && i0 < G.ox1;
+    if (warp == 0) {
+      const float* tab[6] = {a.X.ik, a.X.ad, a.X.b, a.X.ikh, a.X.adh, a.X.bh};
+#pragma unroll
+      for (int q = 0; q < 6; ++q) {
+        float2 t = lact ? *reinterpret_cast<const float2*>(tab[q] + i0) : zero2;
+        if (EDGE && i0 + 1 >= NX) t.y = 0.0f;
+        sts(q * kSC + 2 * lane, t);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < RB; ++j) {
+      const int k = kb + j;
+      vx[j] = vz[j] = sxx[j] = szz[j] = sxz[j] = zero2;
+      float2 c[12];
+#pragma unroll
+      for (int q = 0; q < 12; ++q) c[q] = zero2;
+      if (warp * RB + j < G.R) {
+        const bool zs = EDGE && j < nr && in_strip(k, NZ, W);
+        if (lane == 0) {
+          float* rt = s2_smem + oRT + 8 * j;
+          rt[0] = j < nr ? __ldg(a.Z.ik + k) : 0.0f;
+          rt[1] = j < nr ? __ldg(a.Z.ikh + k) : 0.0f;
+          rt[4] = zs ? __ldg(a.Z.b + k) : 0.0f;
+          rt[5] = zs ? __ldg(a.Z.ad + k) : 0.0f;
+          rt[6] = zs ? __ldg(a.Z.bh + k) : 0.0f;
+          rt[7] = zs ? __ldg(a.Z.adh + k) : 0.0f;
+        }
+        if (j < nr && lact) {
+          const size_t g = (size_t)k * P + i0;
+          vx[j] = *reinterpret_cast<const float2*>(a.vx + g);
+          vz[j] = *reinterpret_cast<const float2*>(a.vz + g);
+          sxx[j] = *reinterpret_cast<const float2*>(a.sxx + g);
+          szz[j] = *reinterpret_cast<const float2*>(a.szz + g);
+          sxz[j] = *reinterpret_cast<const float2*>(a.sxz + g);
+#pragma unroll
+          for (int q = 0; q < 12; ++q) c[q] = *reinterpret_cast<const float2*>(a.coef[q] + g);
+          if (EDGE) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const int i = i0 + e;
+              if (i < 1 || i > NX - 2 || k < 1 || k > NZ - 2) {  // a Dirichlet plane of vx and vz, :365-375
+                el(c[8], e) = el(c[9], e) = 0.0f;
+                plane |= 1u << (2 * j + e);
+              }
+            }
+          }
+          if (k == a.io.sk && a.io.si >= i0 && a.io.si < i0 + 2) src = 2 * j + a.io.si - i0;
+          if (lown && k >= G.oz0 && k < G.oz1) own |= 1u << j;
+        }
+        if (!KEEP)
+#pragma unroll
+          for (int q = 0; q < 12; ++q) sts(oC + j * kRow + q * kSC, c[q]);
+        if (zw) {
+          const bool on = zs && lact;
+          const size_t zg = (size_t)(on ? strip_idx(k, NZ, W) : 0) * P + i0;
+#pragma unroll
+          for (int q = 0; q < 6; ++q)
+            sts(oZ + (6 * j + q) * kSC, on ? *reinterpret_cast<const float2*>(memory[z_index(q)] + zg) : zero2);
+        }
+        if (xsl) {
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const bool on = j < nr && i0 + e < NX && in_strip(i0 + e, NX, W);
+            const size_t xg = on ? (size_t)k * (2 * W) + strip_idx(i0 + e, NX, W) : 0;
+#pragma unroll
+            for (int q = 0; q < 6; ++q) s2_smem[oX + (6 * j + q) * sX + e] = on ? memory[x_index(q)][xg] : 0.0f;
+          }
+        }
+      }
+      if (KEEP)
+#pragma unroll
+        for (int q = 0; q < 12; ++q) keep[KEEP ? j : 0][q] = c[q];
+    }
+  }
+  // ---- receivers of the owned cells: listed by tile, then by thread (a tile
+  // with more than it can list scans the whole list every step instead)
+  for (int q = tid; q < a.io.nrec; q += blockDim.x) {
+    const int i = a.io.rec[3 * q], k = a.io.rec[3 * q + 2];
+    if (i >= G.ox0 && i < G.ox1 && k >= G.oz0 && k < G.oz1) {
+      const int pos = atomicAdd(&G.nrec, 1);
+      if (pos < kResMaxLocalRec) {
+        G.rec[2 * pos] = q;
+        G.rec[2 * pos + 1] = ((k - G.bz) << 6) | (i - G.bx);
+      }
+    }
+  }
+  auto show_v = [&] {  // the velocities the next warps read
+    const int o = kSV + warp * 4 * kSC + 2 * lane;
+    sts(o, vx[0]);
+    sts(o + kSC, vz[0]);
+    sts(o + 2 * kSC, vx[RB - 1]);
+    sts(o + 3 * kSC, vz[RB - 1]);
+  };
+  if (nr > 0) show_v();
+  __syncthreads();
+  int r0 = 0, r1 = 0;  // this thread's entries of G.mine; r1 = -1: scan
+  {
+    const int n = G.nrec;
+    if (n <= kResMaxLocalRec) {
+      auto mine = [&](int q) {
+        const int c = G.rec[2 * q + 1], row = (c >> 6) - warp * RB, col = (c & 63) - 2 * lane;
+        return row >= 0 && row < RB && col >= 0 && col < 2 ? 2 * row + col : -1;
+      };
+      int m = 0;
+      for (int q = 0; q < n; ++q) m += mine(q) >= 0;
+      if (m > 0) {
+        r0 = r1 = atomicAdd(&G.nmine, m);
+        for (int q = 0; q < n; ++q)
+          if (mine(q) >= 0) G.mine[r1++] = G.rec[2 * q] << 4 | mine(q);
+      }
+    } else if (own) {
+      r1 = -1;
+    }
+  }
+
+  // ---- the hand-over: lists as in em2_run_tile, every entry three floats, a
+  // stride apart that its kind tells -- 0 fields (G.hS), 1 z strip (kSC), 2 x
+  // strip (sX)
+  int2* const get = reinterpret_cast<int2*>(s2_smem + G.oGet);
+  int2* const pub = reinterpret_cast<int2*>(s2_smem + G.oPub);
+  const int wz = 2 * NZ * P, wx = wz + 2 * 2 * W * P;
+  const size_t words = (size_t)wx + (size_t)NZ * 2 * 2 * W;
+  unsigned ring = 0;  // owned rows of this lane that lie in a neighbour's halo
+  if (neighbours) {
+    const int htop = G.oz0 - G.bz, hown = G.oz1 - G.oz0, ncols = (G.xend - G.bx + 1) & ~1;
+    const int nB = (htop + G.kend - G.oz1) * kSC;
+    auto strips = [&](int2* list, int* count, int r, int c) {  // the strip words of frame cell (r, c)
+      const int k = G.bz + r, i = G.bx + c;
+      if (EDGE && in_strip(k, NZ, W)) {
+        const int w = r / RB, row = (w < G.wlo ? w : w - G.wh0 + G.wlo) * RB + r % RB;
+        for (int h = 0; h < 2; ++h)
+          list[atomicAdd(count, 1)] =
+              make_int2(wz + s2_word(strip_idx(k, NZ, W), h, i, P), (G.oZ + (6 * row + 3 * h) * kSC + c) | 1 << 28);
+      }
+      if (XS && i < NX && in_strip(i, NX, W)) {
+        const int l = c >> 1, at = G.oX + 6 * r * sX + 2 * (l < G.xlo ? l : l - G.xh0 + G.xlo) + (c & 1);
+        for (int h = 0; h < 2; ++h)
+          list[atomicAdd(count, 1)] =
+              make_int2(wx + (2 * k + h) * 2 * W + strip_idx(i, NX, W), (at + 3 * h * sX) | 2 << 28);
+      }
+    };
+    const int nL = nB + (left ? kS2Halo * hown : 0), nH = nL + (right ? kS2Halo * hown : 0);
+    for (int q = tid; q < nH; q += blockDim.x) {  // the fields first, row by row in the words' order
+      const bool lf = q < nL;
+      const int m = q - (lf ? nB : nL), h = q >> 6;
+      const int r = q < nB ? (h < htop ? h : h + hown) : htop + m / kS2Halo;
+      const int c = q < nB ? ((q & 31) << 1) | ((q >> 5) & 1) : (lf ? 0 : ncols - kS2Halo) + m % kS2Halo;
+      const int slot = q < nB ? h * kSC + c : nB + 2 * kS2Halo * (m / kS2Halo) + (lf ? 0 : kS2Halo) + m % kS2Halo;
+      for (int h2 = 0; h2 < 2; ++h2)
+        get[h2 * nH + q] =
+            c < ncols ? make_int2(s2_word(G.bz + r, h2, G.bx + c, P), G.oH + 3 * h2 * G.hS + slot) : make_int2(-1, 0);
+    }
+    if (tid == 0) G.nget = 2 * nH;
+    __syncthreads();
+    if (EDGE) {
+      for (int q = tid; q < nH; q += blockDim.x) {
+        const bool lf = q < nL;
+        const int m = q - (lf ? nB : nL), h = q >> 6;
+        const int r = q < nB ? (h < htop ? h : h + hown) : htop + m / kS2Halo;
+        const int c = q < nB ? q & 63 : (lf ? 0 : ncols - kS2Halo) + m % kS2Halo;
+        if (c < ncols) strips(get, &G.nget, r, c);
+      }
+    }
+    const int i0 = G.bx + 2 * lane;
+    const bool lring = (left && i0 < G.ox0 + kS2Halo) || (right && i0 >= G.ox1 - kS2Halo);
+#pragma unroll
+    for (int j = 0; j < RB; ++j) {
+      const int r = warp * RB + j, k = G.bz + r;
+      if ((own >> j & 1u) && (lring || (up && k < G.oz0 + kS2Halo) || (down && k >= G.oz1 - kS2Halo))) {
+        ring |= 1u << j;
+        if (EDGE)
+          for (int e = 0; e < 2; ++e) strips(pub, &G.npub, r, 2 * lane + e);
+      }
+    }
+    __syncthreads();
+  }
+  auto hand_over = [&] {  // every thread of the CTA
+    const unsigned tag = G.tag + 1u, want = tag + a.tag_bias;
+    uint4* const word = a.words + (tag & 1u) * words;
+    uint4* const mine = word + s2_word(G.bz + warp * RB, 0, G.bx + 2 * lane, P);
+#pragma unroll
+    for (int j = 0; j < RB; ++j)
+      if (ring >> j & 1u)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          uint4* w = mine + 2 * j * P + e * (P >> 1);
+          st_word(w, el(vx[j], e), el(vz[j], e), el(sxx[j], e), tag);
+          st_word(w + P, el(szz[j], e), el(sxz[j], e), 0.0f, tag);
+        }
+    if (EDGE) {
+      __syncthreads();  // every warp's memory variables are there, and their halo's places are done with
+#pragma unroll 1
+      for (int q = tid; q < G.npub; q += blockDim.x) {
+        const int2 t = pub[q];
+        const float* p = s2_smem + (t.y & 0xfffffff);
+        const int st = t.y >> 28 == 1 ? kSC : sX;
+        st_word(word + t.x, p[0], p[st], p[2 * st], tag);
+      }
+    }
+    unsigned long long t0 = 0;
+    const int n = G.nget;
+#pragma unroll 1
+    for (int q0 = tid; q0 < n; q0 += kS2Batch * blockDim.x) {
+      int2 t[kS2Batch];
+#pragma unroll
+      for (int u = 0; u < kS2Batch; ++u) {
+        const int q = q0 + u * (int)blockDim.x;
+        t[u] = q < n ? get[q] : make_int2(-1, 0);
+      }
+#pragma unroll 1
+      for (int it = 1;; ++it) {
+        uint4 v[kS2Batch];
+#pragma unroll
+        for (int u = 0; u < kS2Batch; ++u)
+          if (t[u].x >= 0) v[u] = ld_word(word + t[u].x);
+        bool more = false;
+#pragma unroll
+        for (int u = 0; u < kS2Batch; ++u) {
+          if (t[u].x < 0) continue;
+          if (v[u].w != want) {
+            more = true;
+            continue;
+          }
+          const int kind = EDGE ? t[u].y >> 28 : 0, st = kind == 0 ? G.hS : kind == 1 ? kSC : sX;
+          float* p = s2_smem + (t[u].y & 0xfffffff);
+          p[0] = __uint_as_float(v[u].x);
+          p[st] = __uint_as_float(v[u].y);
+          p[2 * st] = __uint_as_float(v[u].z);
+          t[u].x = -1;
+        }
+        if (!more) break;
+        if ((it & 15) == 0 && !poll_again(ctl, a.limit_ns, t0)) {
+          G.abort = 1;
+          break;
+        }
+      }
+    }
+    __syncthreads();
+    if (tid == 0) G.tag = tag;
+    // this thread's halo cells
+    const int htop = G.oz0 - G.bz, hown = G.oz1 - G.oz0, i0 = G.bx + 2 * lane, hS = G.hS;
+    if (i0 < G.xend) {
+#pragma unroll
+      for (int j = 0; j < RB; ++j) {
+        const int r = warp * RB + j;
+        if (j >= nr || (own >> j & 1u)) continue;
+        const int o = G.oH + (r < htop           ? r * kSC + 2 * lane
+                              : r >= htop + hown ? (r - hown) * kSC + 2 * lane
+                                                 : hS - 2 * kS2Halo * (htop + hown - r) +
+                                                       (i0 < G.ox0 ? i0 - G.bx : kS2Halo + i0 - G.ox1));
+        vx[j] = lds(o);
+        vz[j] = lds(o + hS);
+        sxx[j] = lds(o + 2 * hS);
+        szz[j] = lds(o + 3 * hS);
+        sxz[j] = lds(o + 4 * hS);
+      }
     }
   };
-  for (int n = tid; n < CS; n += kS2Threads) {
-    int lr, lc;
-    cell_order(n, lr, lc);
-    CELL[n] = (unsigned short)((lr << 7) | lc);
-  }
-  __syncthreads();
-  auto cell_at = [&](int n, int& lr, int& lc) {
-    const unsigned e = CELL[n];
-    lr = (int)(e >> 7);
-    lc = (int)(e & 127u);
-  };
-  auto record = [&](int t) {  // receivers of step t, by the exchange warps
-    float* tr = a.io.traces + (size_t)t * 2 * a.io.nrec;
-    if (nloc <= kResMaxLocalRec) {
-      for (int q = tid; q < nloc; q += 32 * kS2ExchangeWarps) {
-        const int r = s_rec[2 * q], c = s_rec[2 * q + 1];
-        tr[r] = VX[c];
-        tr[a.io.nrec + r] = VZ[c];
+
+  auto coef = [&](int j, int q) { return KEEP ? keep[KEEP ? j : 0][q] : lds(oC + j * kRow + q * kSC); };
+  // b m + ad d: a memory variable's next value
+  auto next = [](float b, float m, float ad, float d) { return __fmaf_rn(b, m, __fmul_rn(ad, d)); };
+  float2 tab[KEEP ? 6 : 1];  // the x tables of this lane
+  if (KEEP)
+#pragma unroll
+    for (int q = 0; q < (KEEP ? 6 : 1); ++q) tab[q] = lds(q * kSC + 2 * lane);
+  auto table = [&](int q) { return KEEP ? tab[KEEP ? q : 0] : lds(q * kSC + 2 * lane); };
+
+  // The stresses of this warp's rows (seismicfdtd.f95:247-312).  ZS: with the
+  // z strip's memory variables (zero tables in the rows outside it)
+  auto stress_rows = [&](auto zs_tag) {
+    constexpr bool ZS = decltype(zs_tag)::value;
+    const int oU = kSV + (max(warp - 1, 0) * 4 + 2) * kSC + 2 * lane, oD = kSV + min(warp + 1, kS2Warps - 1) * 4 * kSC + 2 * lane;
+    const float2 vxt = lds(oU), vzt = lds(oU + kSC), vxb = lds(oD), vzb = lds(oD + kSC);
+    const float2 ikx = table(0), ikxh = table(3);
+    float2 adx, bx, adxh, bxh;
+    if (XS) {
+      adx = table(1);
+      bx = table(2);
+      adxh = table(4);
+      bxh = table(5);
+    }
+#pragma unroll
+    for (int j = 0; j < RB; ++j) {
+      const float2 vxu = j > 0 ? vx[j > 0 ? j - 1 : 0] : vxt, vzu = j > 0 ? vz[j > 0 ? j - 1 : 0] : vzt;
+      const float2 vxd = j < RB - 1 ? vx[j < RB - 1 ? j + 1 : j] : vxb, vzd = j < RB - 1 ? vz[j < RB - 1 ? j + 1 : j] : vzb;
+      const float vxl = __shfl_up_sync(0xffffffffu, vx[j].y, 1), vzl = __shfl_up_sync(0xffffffffu, vz[j].y, 1);
+      const float vxr = __shfl_down_sync(0xffffffffu, vx[j].x, 1), vzr = __shfl_down_sync(0xffffffffu, vz[j].x, 1);
+      const float2 rt = lds(oRT + 8 * j);  // ikz ikzh
+      const float4 zt = ZS ? res::lds4(s2_smem + oRT + 8 * j + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+      // the four differences of either loop: x+ of vx, vz and z- of vz, vx; x- and z+
+      float2 dxx, dzx, dzz, dxz;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        el(dxx, e) = __fsub_rn(e == 0 ? vx[j].y : vxr, el(vx[j], e));
+        el(dzx, e) = __fsub_rn(e == 0 ? vz[j].y : vzr, el(vz[j], e));
+        el(dzz, e) = __fsub_rn(el(vz[j], e), el(vzu, e));
+        el(dxz, e) = __fsub_rn(el(vx[j], e), el(vxu, e));
       }
-    } else {
-      for (int r = tid; r < a.io.nrec; r += 32 * kS2ExchangeWarps) {
-        const int i = a.io.rec[3 * r], k = a.io.rec[3 * r + 2];
-        if (i >= x0 && i < x1 && k >= z0 && k < z1) {
-          tr[r] = VX[fi(k - z0, i - x0)];
-          tr[a.io.nrec + r] = VZ[fi(k - z0, i - x0)];
+      auto gradients = [&](int xm, int zm) {  // scaled, with memory variables xm, xm + 1 of the x strip, zm, zm + 1 of the z strip
+        float2 mxx = zero2, mzx = zero2, mzz = zero2, mxz = zero2;
+        if (XS) {
+          if (xsl) {
+            mxx = lds(oX + (6 * j + xm) * sX);
+            mzx = lds(oX + (6 * j + xm + 1) * sX);
+          }
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            el(mxx, e) = next(el(bxh, e), el(mxx, e), el(adxh, e), el(dxx, e));
+            el(mzx, e) = next(el(bx, e), el(mzx, e), el(adx, e), el(dzx, e));
+          }
+          if (xsl) {
+            sts(oX + (6 * j + xm) * sX, mxx);
+            sts(oX + (6 * j + xm + 1) * sX, mzx);
+          }
+        }
+        if (ZS) {
+          mzz = lds(oZ + (6 * j + zm) * kSC);
+          mxz = lds(oZ + (6 * j + zm + 1) * kSC);
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            el(mzz, e) = next(zt.x, el(mzz, e), zt.y, el(dzz, e));
+            el(mxz, e) = next(zt.z, el(mxz, e), zt.w, el(dxz, e));
+          }
+          sts(oZ + (6 * j + zm) * kSC, mzz);
+          sts(oZ + (6 * j + zm + 1) * kSC, mxz);
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          el(dxx, e) = XS ? __fmaf_rn(el(dxx, e), el(ikxh, e), el(mxx, e)) : __fmul_rn(el(dxx, e), el(ikxh, e));
+          el(dzx, e) = XS ? __fmaf_rn(el(dzx, e), el(ikx, e), el(mzx, e)) : __fmul_rn(el(dzx, e), el(ikx, e));
+          el(dzz, e) = ZS ? __fmaf_rn(el(dzz, e), rt.x, el(mzz, e)) : __fmul_rn(el(dzz, e), rt.x);
+          el(dxz, e) = ZS ? __fmaf_rn(el(dxz, e), rt.y, el(mxz, e)) : __fmul_rn(el(dxz, e), rt.y);
+          el(dzx, e) = __fadd_rn(el(dzx, e), el(dxz, e));  // the shear
+        }
+      };
+      gradients(0, 0);
+      {
+        const float2 A11 = coef(j, 0), A13 = coef(j, 1), A15 = coef(j, 2), A33 = coef(j, 3), A35 = coef(j, 4);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float t = __fmaf_rn(el(A15, e), el(dzx, e), __fmaf_rn(el(A11, e), el(dxx, e), __fmul_rn(el(A13, e), el(dzz, e))));
+          const float u = __fmaf_rn(el(A35, e), el(dzx, e), __fmaf_rn(el(A13, e), el(dxx, e), __fmul_rn(el(A33, e), el(dzz, e))));
+          el(sxx[j], e) = __fadd_rn(el(sxx[j], e), t);
+          el(szz[j], e) = __fadd_rn(el(szz[j], e), u);
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        el(dxx, e) = __fsub_rn(el(vx[j], e), e == 0 ? vxl : vx[j].x);
+        el(dzx, e) = __fsub_rn(el(vz[j], e), e == 0 ? vzl : vz[j].x);
+        el(dzz, e) = __fsub_rn(el(vzd, e), el(vz[j], e));
+        el(dxz, e) = __fsub_rn(el(vxd, e), el(vx[j], e));
+      }
+      gradients(2, 2);
+      {
+        const float2 B15 = coef(j, 5), B35 = coef(j, 6), B55 = coef(j, 7);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float t = __fmaf_rn(el(B55, e), el(dzx, e), __fmaf_rn(el(B15, e), el(dxx, e), __fmul_rn(el(B35, e), el(dzz, e))));
+          el(sxz[j], e) = __fadd_rn(el(sxz[j], e), t);
         }
       }
     }
   };
-  const bool xwarp = warp < kS2ExchangeWarps;
+  // The velocities of this warp's rows (:317-357)
+  auto velocity_rows = [&](auto zs_tag) {
+    constexpr bool ZS = decltype(zs_tag)::value;
+    const float2 sxzt = lds(kSS + (max(warp - 1, 0) * 2 + 1) * kSC + 2 * lane);
+    const float2 szzb = lds(kSS + min(warp + 1, kS2Warps - 1) * 2 * kSC + 2 * lane);
+    const float2 ikx = table(0), ikxh = table(3);
+    float2 adx, bx, adxh, bxh;
+    if (XS) {
+      adx = table(1);
+      bx = table(2);
+      adxh = table(4);
+      bxh = table(5);
+    }
+#pragma unroll
+    for (int j = 0; j < RB; ++j) {
+      const float2 sxzu = j > 0 ? sxz[j > 0 ? j - 1 : 0] : sxzt, szzd = j < RB - 1 ? szz[j < RB - 1 ? j + 1 : j] : szzb;
+      const float sxxl = __shfl_up_sync(0xffffffffu, sxx[j].y, 1), sxzr = __shfl_down_sync(0xffffffffu, sxz[j].x, 1);
+      const float2 rt = lds(oRT + 8 * j);  // ikz ikzh
+      const float4 zt = ZS ? res::lds4(s2_smem + oRT + 8 * j + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+      float2 d1, d2, e1, e2;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        el(d1, e) = __fsub_rn(el(sxx[j], e), e == 0 ? sxxl : sxx[j].x);
+        el(d2, e) = __fsub_rn(el(sxz[j], e), el(sxzu, e));
+        el(e1, e) = __fsub_rn(e == 0 ? sxz[j].y : sxzr, el(sxz[j], e));
+        el(e2, e) = __fsub_rn(el(szzd, e), el(szz[j], e));
+      }
+      float2 m1 = zero2, n1 = zero2;
+      if (XS) {
+        if (xsl) {
+          m1 = lds(oX + (6 * j + 4) * sX);
+          n1 = lds(oX + (6 * j + 5) * sX);
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          el(m1, e) = next(el(bx, e), el(m1, e), el(adx, e), el(d1, e));
+          el(n1, e) = next(el(bxh, e), el(n1, e), el(adxh, e), el(e1, e));
+        }
+        if (xsl) {
+          sts(oX + (6 * j + 4) * sX, m1);
+          sts(oX + (6 * j + 5) * sX, n1);
+        }
+      }
+      if (ZS) {
+        float2 n2 = lds(oZ + (6 * j + 4) * kSC), m2 = lds(oZ + (6 * j + 5) * kSC);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          el(m2, e) = next(zt.x, el(m2, e), zt.y, el(d2, e));
+          el(n2, e) = next(zt.z, el(n2, e), zt.w, el(e2, e));
+        }
+        sts(oZ + (6 * j + 4) * kSC, n2);
+        sts(oZ + (6 * j + 5) * kSC, m2);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          el(d2, e) = __fmaf_rn(el(d2, e), rt.x, el(m2, e));
+          el(e2, e) = __fmaf_rn(el(e2, e), rt.y, el(n2, e));
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          el(d2, e) = __fmul_rn(el(d2, e), rt.x);
+          el(e2, e) = __fmul_rn(el(e2, e), rt.y);
+        }
+      }
+      const float2 rx = coef(j, 8), rz = coef(j, 9);
+      if (a.atten) {
+        const float2 gx = coef(j, 10), gz = coef(j, 11);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          el(vx[j], e) = __fmul_rn(el(vx[j], e), el(gx, e));
+          el(vz[j], e) = __fmul_rn(el(vz[j], e), el(gz, e));
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        float s = __fmaf_rn(el(d1, e), el(ikx, e), el(d2, e)), t = __fmaf_rn(el(e1, e), el(ikxh, e), el(e2, e));
+        if (XS) {
+          s = __fadd_rn(s, el(m1, e));
+          t = __fadd_rn(t, el(n1, e));
+        }
+        el(vx[j], e) = __fmaf_rn(s, el(rx, e), el(vx[j], e));
+        el(vz[j], e) = __fmaf_rn(t, el(rz, e), el(vz[j], e));
+      }
+    }
+  };
+  // add `v0`, `v1`, `v2` to the source cell of f0, f1, f2
+  auto add_at_source = [&](float2* f0, float2* f1, float2* f2, const float* amp, int s) {
+#pragma unroll
+    for (int q = 0; q < 2 * RB; ++q)
+      if (q == src) {
+        el(f0[q / 2], q & 1) += amp[a.t0 + s];
+        el(f1[q / 2], q & 1) += amp[a.io.nstep + a.t0 + s];
+        if (f2) el(f2[q / 2], q & 1) += amp[2 * a.io.nstep + a.t0 + s];
+      }
+  };
 
   float nrm = 0.0f;
-  bool ok = true;
+  const bool rare = src >= 0 || plane || r0 != r1;
   for (int s = 0; s < a.nsteps; ++s) {
-    const int t = a.t0 + s;
-    const int ps = s & 1, pv = (s + 1) & 1;  // parities of the stress and velocity edges
-    const unsigned ts = (unsigned)s + 1u, tv = (unsigned)s + 2u;
-
-    // ================= stresses (seismicfdtd.f95:247-312) on the cell warps;
-    // the exchange warps record the previous step's receivers, then bring in
-    // sxx on the left, sxz on the right and above, szz below
-    if (xwarp) {
-      if (s > 0) record(t - 1);
-      bool good = true;
-      if (warp == 0 && left)
-        good = fetch2(ecol(ps, kESLast, bx - 1) + z0, SXX + fi(0, -1), SW, nullptr, nullptr, 0, tz, ts + a.tag_bias, ctl, a.limit_ns);
-      else if (warp == 1 && right)
-        good = fetch2(ecol(ps, kESFirst, bx + 1) + z0, SXZ + fi(0, tw), SW, nullptr, nullptr, 0, tz, ts + a.tag_bias, ctl, a.limit_ns);
-      else if (warp == 2 && up)
-        good = fetch2(erow(ps, kESLast, bz - 1) + x0, SXZ + fi(-1, 0), 1, nullptr, nullptr, 0, tw, ts + a.tag_bias, ctl, a.limit_ns);
-      else if (warp == 3 && down)
-        good = fetch2(erow(ps, kESFirst, bz + 1) + x0, SZZ + fi(tz, 0), 1, nullptr, nullptr, 0, tw, ts + a.tag_bias, ctl, a.limit_ns);
-      if (!good && (tid & 31) == 0) s_abort = 1;
-    } else {
-      for (int n = tid - 32 * kS2ExchangeWarps; n < CS; n += kS2CellThreads) {
-        int lr, lc;
-        cell_at(n, lr, lc);
-        const int q = lr * tw + lc, k = z0 + lr, i = x0 + lc, f = fi(lr, lc);
-        float sxx = SXX[f], szz = SZZ[f], sxz = SXZ[f];
-        const bool xs = in_strip(i, NX, W), zs = in_strip(k, NZ, W);
-        float mvxx = M[q], mvzz = M[CS + q], mvxz = M[2 * CS + q], mvzx = M[3 * CS + q];
-        // the sigmaxz loop's memory: its own (corrected physics) or loop 1's (legacy)
-        const bool own2 = !a.legacy;
-        const bool loop1 = (k >= 1) && (i <= NX - 2);
-        const bool loop2 = (k <= NZ - 2) && (i >= 1);
-        if (loop1 || loop2) {
-          const float vx0 = VX[f], vz0 = VZ[f];
-          const float ikx = XT[lc], ikxh = XT[3 * tw + lc];
-          const float ikz = ZT[lr], ikzh = ZT[3 * tz + lr];
-          if (loop1) {
-            const float d_vx_x = VX[f + 1] - vx0;
-            const float d_vz_z = vz0 - VZ[f - SW];
-            const float d_vz_x = VZ[f + 1] - vz0;
-            const float d_vx_z = vx0 - VX[f - SW];
-            if (xs) {  // legacy: b_x_half(j), :255 (the q3 row table); corrected: b_x_half(i)
-              mvxx = (a.legacy ? ZT[6 * tz + lr] : XT[5 * tw + lc]) * mvxx + XT[4 * tw + lc] * d_vx_x;
-              mvzx = XT[2 * tw + lc] * mvzx + XT[tw + lc] * d_vz_x;
-            }
-            if (zs) {
-              mvzz = ZT[2 * tz + lr] * mvzz + ZT[tz + lr] * d_vz_z;
-              mvxz = ZT[5 * tz + lr] * mvxz + ZT[4 * tz + lr] * d_vx_z;
-            }
-            const float dvx_dx = d_vx_x * ikxh + mvxx;
-            const float dvz_dz = d_vz_z * ikz + mvzz;
-            const float dvz_dx = d_vz_x * ikx + mvzx;
-            const float dvx_dz = d_vx_z * ikzh + mvxz;
-            const float A11 = C[q], A13 = C[CS + q], A15 = C[2 * CS + q], A33 = C[3 * CS + q], A35 = C[4 * CS + q];
-            const float shear = dvz_dx + dvx_dz;
-            sxx = sxx + (A11 * dvx_dx + A13 * dvz_dz + A15 * shear);
-            szz = szz + (A13 * dvx_dx + A33 * dvz_dz + A35 * shear);
-          }
-          if (loop2) {
-            const float d_vx_x = vx0 - VX[f - 1];
-            const float d_vz_z = VZ[f + SW] - vz0;
-            const float d_vz_x = vz0 - VZ[f - 1];
-            const float d_vx_z = VX[f + SW] - vx0;
-            float mxx = own2 ? M[8 * CS + q] : mvxx, mzz = own2 ? M[9 * CS + q] : mvzz;
-            float mxz = own2 ? M[10 * CS + q] : mvxz, mzx = own2 ? M[11 * CS + q] : mvzx;
-            if (xs) {
-              mxx = XT[5 * tw + lc] * mxx + XT[4 * tw + lc] * d_vx_x;
-              mzx = XT[2 * tw + lc] * mzx + XT[tw + lc] * d_vz_x;
-            }
-            if (zs) {
-              mzz = ZT[2 * tz + lr] * mzz + ZT[tz + lr] * d_vz_z;
-              mxz = ZT[5 * tz + lr] * mxz + ZT[4 * tz + lr] * d_vx_z;
-            }
-            const float dvx_dx = d_vx_x * ikxh + mxx;
-            const float dvz_dz = d_vz_z * ikz + mzz;
-            const float dvz_dx = d_vz_x * ikx + mzx;
-            const float dvx_dz = d_vx_z * ikzh + mxz;
-            sxz = sxz + (C[5 * CS + q] * dvx_dx + C[6 * CS + q] * dvz_dz + C[7 * CS + q] * (dvz_dx + dvx_dz));
-            if (own2) {
-              if (xs) { M[8 * CS + q] = mxx; M[11 * CS + q] = mzx; }
-              if (zs) { M[9 * CS + q] = mzz; M[10 * CS + q] = mxz; }
-            } else {
-              mvxx = mxx; mvzz = mzz; mvxz = mxz; mvzx = mzx;
-            }
-          }
-          if (a.io.ssrc && i == si && k == sk) {  // stress source: sigma_ij += f_ij(t) dt
-            sxx += a.io.ssrc[t];
-            szz += a.io.ssrc[a.io.nstep + t];
-            sxz += a.io.ssrc[2 * a.io.nstep + t];
-          }
-          SXX[f] = sxx;
-          SZZ[f] = szz;
-          SXZ[f] = sxz;
-          if (xs) {
-            M[q] = mvxx;
-            M[3 * CS + q] = mvzx;
-          }
-          if (zs) {
-            M[CS + q] = mvzz;
-            M[2 * CS + q] = mvxz;
-          }
-        }
-        if (right && lc == tw - 1) ll_put1(ecol(ps, kESLast, bx) + k, sxx, ts);
-        if (left && lc == 0) ll_put1(ecol(ps, kESFirst, bx) + k, sxz, ts);
-        if (down && lr == tz - 1) ll_put1(erow(ps, kESLast, bz) + i, sxz, ts);
-        if (up && lr == 0) ll_put1(erow(ps, kESFirst, bz) + i, szz, ts);
-      }
+    // a run with no hand-over in it has one before it, so that no tile writes
+    // back what a neighbour has yet to load
+    if (neighbours && (s > 0 ? s % kS2Steps == 0 : a.nsteps <= kS2Steps)) {
+      hand_over();
+      if (G.abort) return;  // the state is left as it was loaded; the host reports the timeout
+      if (nr > 0) show_v();
+      __syncthreads();
+    }
+    if (nr > 0) {
+      if (zw) stress_rows(std::true_type{});
+      else stress_rows(std::false_type{});
+      if (src >= 0 && a.io.ssrc) add_at_source(sxx, szz, sxz, a.io.ssrc, s);  // sigma_ij += f_ij(t) dt
+      sts(kSS + warp * 2 * kSC + 2 * lane, szz[0]);
+      sts(kSS + (warp * 2 + 1) * kSC + 2 * lane, sxz[RB - 1]);
     }
     __syncthreads();
-    if (s_abort) {
-      ok = false;
-      break;
-    }
-
-    // ================= velocities, source, Dirichlet planes, norm (:317-379)
-    // on the cell warps; the exchange warps bring in the velocity halo of the
-    // next step
-    if (xwarp) {
-      bool good = true;
-      if (s + 1 < a.nsteps) {
-        if (warp == 0 && left)
-          good = fetch2(ecol(pv, kEVxLast, bx - 1) + z0, VX + fi(0, -1), SW, ecol(pv, kEVzLast, bx - 1) + z0,
-                        VZ + fi(0, -1), SW, tz, tv + a.tag_bias, ctl, a.limit_ns);
-        else if (warp == 1 && right)
-          good = fetch2(ecol(pv, kEVxFirst, bx + 1) + z0, VX + fi(0, tw), SW, ecol(pv, kEVzFirst, bx + 1) + z0,
-                        VZ + fi(0, tw), SW, tz, tv + a.tag_bias, ctl, a.limit_ns);
-        else if (warp == 2 && up)
-          good = fetch2(erow(pv, kEVxLast, bz - 1) + x0, VX + fi(-1, 0), 1, erow(pv, kEVzLast, bz - 1) + x0,
-                        VZ + fi(-1, 0), 1, tw, tv + a.tag_bias, ctl, a.limit_ns);
-        else if (warp == 3 && down)
-          good = fetch2(erow(pv, kEVxFirst, bz + 1) + x0, VX + fi(tz, 0), 1, erow(pv, kEVzFirst, bz + 1) + x0,
-                        VZ + fi(tz, 0), 1, tw, tv + a.tag_bias, ctl, a.limit_ns);
-      }
-      if (!good && (tid & 31) == 0) s_abort = 1;
-    } else {
-      for (int n = tid - 32 * kS2ExchangeWarps; n < CS; n += kS2CellThreads) {
-        int lr, lc;
-        cell_at(n, lr, lc);
-        const int q = lr * tw + lc, k = z0 + lr, i = x0 + lc, f = fi(lr, lc);
-        const bool xs = in_strip(i, NX, W), zs = in_strip(k, NZ, W);
-        const bool interior = (i >= 1) && (i <= NX - 2) && (k >= 1) && (k <= NZ - 2);
-        float vx = 0.f, vz = 0.f;
-        if (k >= 1 && i >= 1) {  // vx loop, :317-336
-          const float d1 = SXX[f] - SXX[f - 1];
-          const float d2 = SXZ[f] - SXZ[f - SW];
-          float v1 = d1 * XT[lc], v2 = d2 * ZT[lr];
-          if (xs) {
-            const float m = XT[2 * tw + lc] * M[4 * CS + q] + XT[tw + lc] * d1;
-            M[4 * CS + q] = m;
-            v1 += m;
+    if (nr > 0) {
+      if (zw) velocity_rows(std::true_type{});
+      else velocity_rows(std::false_type{});
+      if (rare) {
+        if (src >= 0) add_at_source(vx, vz, nullptr, a.io.src, s);  // :360-361
+        if (EDGE && plane) {  // :365-375
+#pragma unroll
+          for (int q = 0; q < 2 * RB; ++q)
+            if (plane >> q & 1u) el(vx[q / 2], q & 1) = el(vz[q / 2], q & 1) = 0.0f;
+        }
+        if (r0 != r1) {  // receivers of step t
+          float* tr = a.io.traces + (size_t)(a.t0 + s) * 2 * a.io.nrec;
+          auto sample = [&](int r, int c) {  // cell c = 2 * row + element
+            float x = 0.0f, z = 0.0f;
+#pragma unroll
+            for (int q = 0; q < 2 * RB; ++q)
+              if (q == c) {
+                x = el(vx[q / 2], q & 1);
+                z = el(vz[q / 2], q & 1);
+              }
+            tr[r] = x;
+            tr[a.io.nrec + r] = z;
+          };
+          if (r1 >= 0) {
+            for (int q = r0; q < r1; ++q) sample(G.mine[q] >> 4, G.mine[q] & 15);
+          } else {
+            const int i0 = G.bx + 2 * lane, kb = G.bz + warp * RB;
+            for (int q = 0; q < a.io.nrec; ++q) {
+              const int e = a.io.rec[3 * q] - i0, j = a.io.rec[3 * q + 2] - kb;
+              if (e >= 0 && e < 2 && j >= 0 && j < RB && (own >> j & 1u)) sample(q, 2 * j + e);
+            }
           }
-          if (zs) {
-            const float m = ZT[2 * tz + lr] * M[7 * CS + q] + ZT[tz + lr] * d2;
-            M[7 * CS + q] = m;
-            v2 += m;
-          }
-          if (interior) {
-            vx = VX[f];
-            if (a.atten) vx *= C[10 * CS + q];
-            vx = vx + (v1 + v2) * C[8 * CS + q];
-          }
-        }
-        if (k <= NZ - 2 && i <= NX - 2) {  // vz loop, :338-357
-          const float d1 = SXZ[f + 1] - SXZ[f];
-          const float d2 = SZZ[f + SW] - SZZ[f];
-          float v1 = d1 * XT[3 * tw + lc], v2 = d2 * ZT[3 * tz + lr];
-          if (xs) {
-            const float m = XT[5 * tw + lc] * M[6 * CS + q] + XT[4 * tw + lc] * d1;
-            M[6 * CS + q] = m;
-            v1 += m;
-          }
-          if (zs) {
-            const float m = ZT[5 * tz + lr] * M[5 * CS + q] + ZT[4 * tz + lr] * d2;
-            M[5 * CS + q] = m;
-            v2 += m;
-          }
-          if (interior) {
-            vz = VZ[f];
-            if (a.atten) vz *= C[11 * CS + q];
-            vz = vz + (v1 + v2) * C[9 * CS + q];
-          }
-        }
-        if (i == si && k == sk) {  // :360-361
-          vx += a.io.src[t];
-          vz += a.io.src[a.io.nstep + t];
-        }
-        if (!interior) {  // :365-375
-          vx = 0.f;
-          vz = 0.f;
-        }
-        VX[f] = vx;
-        VZ[f] = vz;
-        nrm = fmaxf(nrm, norm_monitor(vx, vz));
-        if (left && lc == 0) {
-          ll_put1(ecol(pv, kEVxFirst, bx) + k, vx, tv);
-          ll_put1(ecol(pv, kEVzFirst, bx) + k, vz, tv);
-        }
-        if (right && lc == tw - 1) {
-          ll_put1(ecol(pv, kEVxLast, bx) + k, vx, tv);
-          ll_put1(ecol(pv, kEVzLast, bx) + k, vz, tv);
-        }
-        if (up && lr == 0) {
-          ll_put1(erow(pv, kEVxFirst, bz) + i, vx, tv);
-          ll_put1(erow(pv, kEVzFirst, bz) + i, vz, tv);
-        }
-        if (down && lr == tz - 1) {
-          ll_put1(erow(pv, kEVxLast, bz) + i, vx, tv);
-          ll_put1(erow(pv, kEVzLast, bz) + i, vz, tv);
         }
       }
+      if (own) {  // the norm monitor: |vx| + |vz| of the owned cells
+        float big = 0.0f;
+#pragma unroll
+        for (int j = 0; j < RB; ++j)
+          if (own >> j & 1u)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) big = max_nan(big, fabsf(el(vx[j], e)) + fabsf(el(vz[j], e)));
+        if (big <= 1e24f) {
+          nrm = fmaxf(nrm, big);
+        } else {  // near the threshold, or NaN: the 2-norm itself
+          float sq = 0.0f;
+#pragma unroll
+          for (int j = 0; j < RB; ++j)
+            if (own >> j & 1u)
+#pragma unroll
+              for (int e = 0; e < 2; ++e) sq = max_nan(sq, norm_sq(el(vx[j], e), el(vz[j], e)));
+          nrm = fmaxf(nrm, norm_of_sq(sq));
+        }
+      }
+      if (DUMP && own) {  // the state after step t into slot s + 1 (streaming stores: read once, by the adjoint)
+        char* slot = a.dump.base + a.dump.stride * (size_t)(s + 1);
+        auto arr = [&](int q) { return reinterpret_cast<float*>(slot + a.dump.off[q]); };
+        const int i0 = G.bx + 2 * lane, kb = G.bz + warp * RB;
+#pragma unroll
+        for (int j = 0; j < RB; ++j) {
+          const int k = kb + j;
+          if (!(own >> j & 1u)) continue;
+          const size_t g = (size_t)k * P + i0;
+          __stcs(reinterpret_cast<float2*>(arr(0) + g), vx[j]);
+          __stcs(reinterpret_cast<float2*>(arr(1) + g), vz[j]);
+          __stcs(reinterpret_cast<float2*>(arr(2) + g), sxx[j]);
+          __stcs(reinterpret_cast<float2*>(arr(3) + g), szz[j]);
+          __stcs(reinterpret_cast<float2*>(arr(4) + g), sxz[j]);
+          if (EDGE && in_strip(k, NZ, W)) {
+            const size_t zg = (size_t)strip_idx(k, NZ, W) * P + i0;
+#pragma unroll
+            for (int q = 0; q < 6; ++q) {
+              float2 m = lds(oZ + (6 * j + q) * kSC);
+#pragma unroll
+              for (int e = 0; e < 2; ++e)
+                if (i0 + e >= NX || !in_loop(true, q, i0 + e, k, NX, NZ)) el(m, e) = 0.0f;
+              __stcs(reinterpret_cast<float2*>(arr(5 + z_index(q)) + zg), m);
+            }
+          }
+          if (xsl) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+              if (i0 + e < NX && in_strip(i0 + e, NX, W)) {
+                const size_t xg = (size_t)k * (2 * W) + strip_idx(i0 + e, NX, W);
+#pragma unroll
+                for (int q = 0; q < 6; ++q)
+                  __stcs(arr(5 + x_index(q)) + xg,
+                         in_loop(false, q, i0 + e, k, NX, NZ) ? s2_smem[oX + (6 * j + q) * sX + e] : 0.0f);
+              }
+          }
+        }
+      }
+      show_v();
     }
     __syncthreads();
-    if (s_abort) {
-      ok = false;
-      break;
-    }
-    if (DUMP) {  // the state after step t into slot s + 1 (streaming stores: read once, by the adjoint)
-      char* slot = a.dump.base + a.dump.stride * (size_t)(s + 1);
-      auto arr = [&](int q) { return reinterpret_cast<float*>(slot + a.dump.off[q]); };
-      for (int q = tid; q < CS; q += kS2Threads) {
-        const int lr = q / tw, lc = q - lr * tw, k = z0 + lr, i = x0 + lc, f = fi(lr, lc);
-        const size_t g = (size_t)k * P + i;
-        __stcs(arr(0) + g, VX[f]);
-        __stcs(arr(1) + g, VZ[f]);
-        __stcs(arr(2) + g, SXX[f]);
-        __stcs(arr(3) + g, SZZ[f]);
-        __stcs(arr(4) + g, SXZ[f]);
-        if (in_strip(i, NX, W)) {
-          const size_t mx = (size_t)k * (2 * W) + strip_idx(i, NX, W);
-          const int xm[6] = {0, 3, 4, 6, 8, 11};
-#pragma unroll
-          for (int e = 0; e < 6; ++e) __stcs(arr(5 + xm[e]) + mx, M[xm[e] * CS + q]);
-        }
-        if (in_strip(k, NZ, W)) {
-          const size_t mz = (size_t)strip_idx(k, NZ, W) * P + i;
-          const int zm[6] = {1, 2, 5, 7, 9, 10};
-#pragma unroll
-          for (int e = 0; e < 6; ++e) __stcs(arr(5 + zm[e]) + mz, M[zm[e] * CS + q]);
-        }
-      }
-      __syncthreads();  // the next step's stresses overwrite what the dump reads
-    }
-  }
-  if (ok && xwarp && a.nsteps > 0) record(a.t0 + a.nsteps - 1);
-  if (!ok) return;  // the state is left as it was loaded; the host reports the timeout
-  if (DUMP) {
-    block_norm_to_slot(nrm, a.io.slots, blockIdx.x);
-    return;
   }
 
-  // ---- write the tile back
-  for (int q = tid; q < CS; q += kS2Threads) {
-    const int lr = q / tw, lc = q - lr * tw, k = z0 + lr, i = x0 + lc, f = fi(lr, lc);
-    const size_t g = (size_t)k * P + i;
-    a.vx[g] = VX[f];
-    a.vz[g] = VZ[f];
-    a.sxx[g] = SXX[f];
-    a.szz[g] = SZZ[f];
-    a.sxz[g] = SXZ[f];
-    if (in_strip(i, NX, W)) {
-      const size_t mx = (size_t)k * (2 * W) + strip_idx(i, NX, W);
-      a.m_vxx[mx] = M[q];
-      a.m_vzx[mx] = M[3 * CS + q];
-      a.m_sxx_x[mx] = M[4 * CS + q];
-      a.m_sxz_x[mx] = M[6 * CS + q];
-      if (!a.legacy) {
-        a.m2_vxx[mx] = M[8 * CS + q];
-        a.m2_vzx[mx] = M[11 * CS + q];
+  // ---- write the owned cells back (a recompute for the adjoint keeps its input)
+  if (!DUMP && own) {
+    const int i0 = G.bx + 2 * lane, kb = G.bz + warp * RB;
+#pragma unroll
+    for (int j = 0; j < RB; ++j) {
+      const int k = kb + j;
+      if (!(own >> j & 1u)) continue;
+      const size_t g = (size_t)k * P + i0;
+      *reinterpret_cast<float2*>(a.vx + g) = vx[j];
+      *reinterpret_cast<float2*>(a.vz + g) = vz[j];
+      *reinterpret_cast<float2*>(a.sxx + g) = sxx[j];
+      *reinterpret_cast<float2*>(a.szz + g) = szz[j];
+      *reinterpret_cast<float2*>(a.sxz + g) = sxz[j];
+      if (EDGE && in_strip(k, NZ, W)) {
+        const size_t zg = (size_t)strip_idx(k, NZ, W) * P + i0;
+#pragma unroll
+        for (int q = 0; q < 6; ++q)
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+            if (i0 + e < NX && in_loop(true, q, i0 + e, k, NX, NZ))
+              memory[z_index(q)][zg + e] = s2_smem[oZ + (6 * j + q) * kSC + e];
       }
-    }
-    if (in_strip(k, NZ, W)) {
-      const size_t mz = (size_t)strip_idx(k, NZ, W) * P + i;
-      a.m_vzz[mz] = M[CS + q];
-      a.m_vxz[mz] = M[2 * CS + q];
-      a.m_szz_z[mz] = M[5 * CS + q];
-      a.m_sxz_z[mz] = M[7 * CS + q];
-      if (!a.legacy) {
-        a.m2_vzz[mz] = M[9 * CS + q];
-        a.m2_vxz[mz] = M[10 * CS + q];
+      if (xsl) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          if (i0 + e < NX && in_strip(i0 + e, NX, W)) {
+            const size_t xg = (size_t)k * (2 * W) + strip_idx(i0 + e, NX, W);
+#pragma unroll
+            for (int q = 0; q < 6; ++q)
+              if (in_loop(false, q, i0 + e, k, NX, NZ)) memory[x_index(q)][xg] = s2_smem[oX + (6 * j + q) * sX + e];
+          }
       }
     }
   }
   block_norm_to_slot(nrm, a.io.slots, blockIdx.x);
 }
 
-}  // namespace
-
-bool seis2_resident_plan(int NX, int NZ, int max_ctas, size_t max_smem, Seis2ResPlan* out) {
-  max_ctas = std::min(max_ctas, kResMaxTiles);
-  long best = -1;
-  int bnx = 0, bnz = 0;
-  for (int ntz = 1; ntz <= std::min(kResMaxTiles1D, NZ); ++ntz)
-    for (int ntx = 1; ntx <= std::min(kResMaxTiles1D, NX) && ntx * ntz <= max_ctas; ++ntx) {
-      const int TW = (NX + ntx - 1) / ntx, TZ = (NZ + ntz - 1) / ntz;
-      if (TW > kS2MaxTile || TZ > kS2MaxTile || s2_smem(TW, TZ) > max_smem) continue;
-      // the largest tile sets the pace; among equals, the shorter perimeter
-      const long cost = 4L * TW * TZ + TW + TZ;
-      if (best < 0 || cost < best) {
-        best = cost;
-        bnx = ntx;
-        bnz = ntz;
-      }
-    }
-  if (best < 0) return false;
-  out->ntx = bnx;
-  out->ntz = bnz;
-  for (int c = 0; c <= bnx; ++c) out->xb[c] = (int)((long)c * NX / bnx);
-  for (int r = 0; r <= bnz; ++r) out->zb[r] = (int)((long)r * NZ / bnz);
-  out->smem = s2_smem((NX + bnx - 1) / bnx, (NZ + bnz - 1) / bnz);
-  return true;
+template <int RB, bool DUMP>
+__global__ void __launch_bounds__(32 * kS2Warps, 1) seis2_resident_kernel(const __grid_constant__ Seis2Resident a) {
+  __shared__ S2Tile G;
+  const int kind = a.tiles.tile[blockIdx.x].z;
+  if (kind == 0) s2_run_tile<RB, DUMP, false, false>(a, G);
+  else if (kind == 1) s2_run_tile<RB, DUMP, true, false>(a, G);
+  else s2_run_tile<RB, DUMP, true, true>(a, G);
 }
 
-cudaError_t seis2_resident_prepare(const Seis2ResPlan& plan, int* ctas_per_sm) {
-  const void* fns[2] = {(const void*)seis2_resident_kernel<false>, (const void*)seis2_resident_kernel<true>};
+const void* s2_kernel(int rb, bool dump) {
+  static const void* const k[kS2MaxRows][2] = {
+      {(const void*)seis2_resident_kernel<1, false>, (const void*)seis2_resident_kernel<1, true>},
+      {(const void*)seis2_resident_kernel<2, false>, (const void*)seis2_resident_kernel<2, true>},
+      {(const void*)seis2_resident_kernel<3, false>, (const void*)seis2_resident_kernel<3, true>}};
+  return k[rb - 1][dump];
+}
+
+// Shared memory of a frame with rb rows a warp, as s2_run_tile lays it out.
+size_t s2_tile_smem(const Frame& f, int rb) {
+  const size_t R = (size_t)(f.rows + rb - 1) / rb * rb;
+  const int hrows = f.rows - f.own;
+  const int zn = f.edge ? f.zlo + f.zhi : 0, xl = f.edge ? f.xlanes : 0;
+  size_t n = kSCo + (rb <= kS2Keep ? 0 : 12 * kSC * R) + 6 * ((size_t)hrows * kSC + 2 * kS2Halo * (size_t)f.own) + 1 +
+             2 * (size_t)(s2_get_entries(hrows, f.own, zn, xl) + s2_pub_entries(f.own, zn, xl));
+  if (f.edge) {
+    const size_t wlo = (f.zlo + rb - 1) / rb, wh0 = std::max<size_t>(f.zhi0 / rb, wlo);
+    n += 6 * kSC * rb * (wlo + (R / rb > wh0 ? R / rb - wh0 : 0)) + 12 * R * (size_t)f.xlanes;
+  }
+  return sizeof(float) * n;
+}
+
+// The planner's cost model (tile_plan.h).
+#ifndef SFD_S2_ZROW_COST
+#define SFD_S2_ZROW_COST 0.7
+#endif
+#ifndef SFD_S2_XCOL_COST
+#define SFD_S2_XCOL_COST 0.5
+#endif
+#ifndef SFD_S2_MIN_COST
+#define SFD_S2_MIN_COST 16.0
+#endif
+
+}  // namespace
+
+bool seis2_resident_plan(int NX, int NZ, int npml, int max_ctas, size_t max_smem, TilePlan* out) {
+  const TileRules rules{2, kS2Halo, kS2MaxRows, kS2Warps, SFD_S2_ZROW_COST, SFD_S2_XCOL_COST, SFD_S2_MIN_COST};
+  return plan_tiles(rules, NX, NZ, npml, max_ctas, max_smem, s2_tile_smem, out);
+}
+
+cudaError_t seis2_resident_prepare(const TilePlan& plan, int* ctas_per_sm) {
   int n = 1 << 30;
-  for (const void* fn : fns) {
+  for (int dump = 0; dump < 2; ++dump) {
+    const void* fn = s2_kernel(plan.rb, dump);
     cudaError_t e = res_allow_max_smem(fn);
     int q = 0;
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&q, fn, kS2Threads, plan.smem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&q, fn, 32 * plan.warps, plan.smem);
     if (e != cudaSuccess) return e;
     n = std::min(n, q);
   }
@@ -583,8 +837,8 @@ cudaError_t seis2_resident_prepare(const Seis2ResPlan& plan, int* ctas_per_sm) {
 
 cudaError_t seis2_resident_launch(const Seis2Resident& a, cudaStream_t s) {
   void* args[] = {(void*)&a};
-  const void* fn = a.dump.base ? (const void*)seis2_resident_kernel<true> : (const void*)seis2_resident_kernel<false>;
-  return cudaLaunchCooperativeKernel(fn, dim3(a.plan.ntx * a.plan.ntz), dim3(kS2Threads), args, a.plan.smem, s);
+  return cudaLaunchCooperativeKernel(s2_kernel(a.tiles.rb, a.dump.base != nullptr), dim3(a.tiles.ntiles),
+                                     dim3(32 * a.tiles.warps), args, a.tiles.smem, s);
 }
 
 }  // namespace sfd

@@ -244,13 +244,11 @@ int s2_adjoint_segment(sfd_handle* h, int64_t nsteps, bool recorded, int64_t s0)
     int r = s2_save_state(h, A, h->adj + A.slots);
     if (r) return r;
   }
-  begin_run(h, s0);
   const bool on_chip = recorded || resident_usable(h);
+  begin_run(h, s0, on_chip && !recorded ? s2_hand_overs((int)nsteps) : 0);
   if (on_chip && !recorded) {  // the recompute as one on-chip launch that writes every step's state into its slot
-    const Layout& L = h->L;
     Seis2Resident fr = s2_dump_args(h, A, s0, nsteps);
     fr.io.nrec = 0;
-    CK(cudaMemsetAsync(h->base + L.off_res, 0, res_scratch_bytes(L.P, L.NZ, res_edge_fields(h->cfg.kind)), h->stream));
     CK(seis2_resident_launch(fr, h->stream));
   }
   if (!h->cap_stream) {
@@ -572,8 +570,7 @@ int32_t sfd_adjoint_record(sfd_handle* h, int64_t nsteps) {
     const Layout& L = h->L;
     r = s2_save_state(h, A, h->adj + A.slots);
     if (r) return r;
-    begin_run(h, h->step);
-    CK(cudaMemsetAsync(h->base + L.off_res, 0, res_scratch_bytes(L.P, L.NZ, res_edge_fields(h->cfg.kind)), h->stream));
+    begin_run(h, h->step, s2_hand_overs((int)nsteps));
     const Seis2Resident own = seis2_resident_args(h, nsteps);
     CK(seis2_resident_launch(s2_dump_args(h, A, h->step, nsteps), h->stream));  // receivers recorded as in sfd_run
     reduce_norms(h);

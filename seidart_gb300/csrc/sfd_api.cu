@@ -190,6 +190,7 @@ bool pingpong_mem(int kind, int q) {
 }
 bool has_single_pass(int kind) { return kind == SFD_ELECTROMAG2 || kind == SFD_SEISMIC2; }
 bool cpml2d(const sfd_config& c) { return (c.flags & SFD_FLAG_CPML_2D) != 0; }
+bool legacy_quirks(const sfd_config& c) { return (c.flags & SFD_FLAG_LEGACY_QUIRKS) != 0; }
 // Whether a handle steps in the single-pass form (the others: two kernels per step).
 bool single_pass(const sfd_config& c) {
   return has_single_pass(c.kind) && !(c.flags & (SFD_FLAG_TWO_PASS | SFD_FLAG_CPML_2D));
@@ -272,14 +273,16 @@ void make_layout(const sfd_config& c, Layout* L) {
   L->off_traces = o; o += align256(sizeof(float) * (size_t)c.nstep * nchan(c.kind) * std::max(1, c.nrec));
   L->off_slots = o; o += align256(sizeof(float) * L->nslots);  // ZB = 1 tiles: the largest grid
   L->off_res = 0;
-  if (single_pass(c) && !(c.flags & SFD_FLAG_STREAMING)) {
-    L->off_res = o;  // edge arrays of on-chip runs
+  const bool on_chip = single_pass(c) && !(c.flags & SFD_FLAG_STREAMING);
+  if (on_chip && (c.kind == SFD_ELECTROMAG2 || legacy_quirks(c))) {
+    L->off_res = o;  // edge arrays of the on-chip electromag2 adjoint sweep and of the legacy quirks' run
     o += align256(res_scratch_bytes(L->P, c.nz, res_edge_fields(c.kind)));
   }
   L->off_words = 0;
-  if (L->off_res && c.kind == SFD_ELECTROMAG2 && (size_t)L->P * c.nz <= kEm2MaxCells) {
+  const bool em2 = c.kind == SFD_ELECTROMAG2;
+  if (on_chip && !legacy_quirks(c) && (size_t)L->P * c.nz <= (em2 ? kEm2MaxCells : kS2MaxCells)) {
     L->off_words = o;  // hand-over words of on-chip runs
-    o += align256(em2_word_bytes(L->P, c.nz, c.npml));
+    o += align256(em2 ? em2_word_bytes(L->P, c.nz, c.npml) : s2_word_bytes(L->P, c.nz, c.npml));
   }
   L->total = o;
 }
@@ -520,7 +523,7 @@ void launch_finalize(sfd_handle* h, int t_last, cudaStream_t s) {
 bool resident_usable(sfd_handle* h) {
   if (h->res_state) return h->res_state > 0;
   h->res_state = -1;
-  if (!h->L.off_res || !h->single) return false;
+  if ((!h->L.off_words && !(h->L.off_res && legacy_quirks(h->cfg))) || !h->single) return false;
   int dev = 0, nsm = 0, coop = 0, optin = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
@@ -530,30 +533,24 @@ bool resident_usable(sfd_handle* h) {
     return false;
   }
   if (!coop) return false;
-  const size_t static_smem = 8192;  // receiver list, thread map and reduction buffers of the kernel
-  if (h->cfg.kind == SFD_SEISMIC2) {  // a uniform tiling: searched in microseconds, not cached
-    Seis2ResPlan plan;
-    if (!seis2_resident_plan(h->cfg.nx, h->cfg.nz, std::min(nsm, h->L.nslots), (size_t)optin - static_smem, &plan))
-      return false;
-    int per_sm = 0;
-    if (seis2_resident_prepare(plan, &per_sm) != cudaSuccess || per_sm < 1) {
-      cudaGetLastError();
-      return false;
-    }
-    h->s2_plan = plan;
-    h->res_state = 1;
-    return true;
-  }
-  if (!h->L.off_words) return false;
-  Em2Plan plan;  // searched in tens of microseconds, not cached
-  if (!em2_resident_plan(h->cfg.nx, h->cfg.nz, h->cfg.npml, std::min(nsm, h->L.nslots), (size_t)optin - static_smem, &plan))
-    return false;
+  const size_t static_smem = 8192;  // the kernels' static shared memory (receiver lists, reduction buffers)
+  const int ctas = std::min(nsm, h->L.nslots);
+  const size_t smem = (size_t)optin - static_smem;
+  const sfd_config& c = h->cfg;
   int per_sm = 0;
-  if (em2_resident_prepare(plan, &per_sm) != cudaSuccess || per_sm < 1) {
+  bool fits;  // the tilings are searched in tens of microseconds, not cached
+  if (legacy_quirks(c))
+    fits = seis2_legacy_plan(c.nx, c.nz, ctas, smem, &h->s2_plan) && seis2_legacy_prepare(h->s2_plan, &per_sm) == cudaSuccess;
+  else if (c.kind == SFD_SEISMIC2)
+    fits = seis2_resident_plan(c.nx, c.nz, c.npml, ctas, smem, &h->res_plan) &&
+           seis2_resident_prepare(h->res_plan, &per_sm) == cudaSuccess;
+  else
+    fits = em2_resident_plan(c.nx, c.nz, c.npml, ctas, smem, &h->res_plan) &&
+           em2_resident_prepare(h->res_plan, &per_sm) == cudaSuccess;
+  if (!fits || per_sm < 1) {
     cudaGetLastError();
     return false;
   }
-  h->res_plan = plan;
   h->res_state = 1;
   return true;
 }
@@ -625,6 +622,8 @@ Seis2Resident seis2_resident_args(const sfd_handle* h, int64_t nsteps) {
   r.q3 = b.q3;
   r.X = b.X; r.Z = b.Z;
   r.io = b.io;
+  r.tiles = h->res_plan;
+  r.words = (uint4*)(h->base + h->L.off_words);
   r.plan = h->s2_plan;
   char* base = h->base + h->L.off_res;
   r.r.erow = (uint2*)base;
@@ -1540,13 +1539,15 @@ int32_t sfd_run(sfd_handle* h, int64_t nsteps) {
   Ctl* ctl = (Ctl*)(h->base + L.off_ctl);
   float* slots = (float*)(h->base + L.off_slots);
   const bool on_chip = resident_usable(h), em2 = h->cfg.kind == SFD_ELECTROMAG2;
-  begin_run(h, h->step, on_chip && em2 ? em2_hand_overs((int)nsteps) : 0);
+  begin_run(h, h->step, !on_chip ? 0 : em2 ? em2_hand_overs((int)nsteps) : s2_hand_overs((int)nsteps));
   if (on_chip) {  // the whole run in one launch, state on chip
     if (em2) {
       CK(em2_resident_launch(resident_args(h, nsteps), h->stream));
-    } else {
+    } else if (legacy_quirks(h->cfg)) {
       // tags from an earlier run must not match: clear every edge word
       CK(cudaMemsetAsync(h->base + L.off_res, 0, res_scratch_bytes(L.P, L.NZ, res_edge_fields(h->cfg.kind)), h->stream));
+      CK(seis2_legacy_launch(seis2_resident_args(h, nsteps), h->stream));
+    } else {
       CK(seis2_resident_launch(seis2_resident_args(h, nsteps), h->stream));
     }
     k_reduce_slots<<<1, 1024, 0, h->stream>>>(ctl, slots, L.nslots);
@@ -1581,9 +1582,9 @@ int32_t sfd_on_chip(sfd_handle* h, int32_t* tiles_x, int32_t* tiles_z) {  // til
   g_err.clear();
   if (!h) return fail(SFD_ERR_BAD_ARG, "NULL handle");
   const bool on = resident_usable(h);
-  const bool s2 = h->cfg.kind == SFD_SEISMIC2;
-  if (tiles_x) *tiles_x = on ? (s2 ? h->s2_plan.ntx * h->s2_plan.ntz : h->res_plan.ntiles) : 0;
-  if (tiles_z) *tiles_z = on ? (s2 ? h->s2_plan.ntz : h->res_plan.ntz) : 0;
+  const bool legacy = legacy_quirks(h->cfg);
+  if (tiles_x) *tiles_x = on ? (legacy ? h->s2_plan.ntx * h->s2_plan.ntz : h->res_plan.ntiles) : 0;
+  if (tiles_z) *tiles_z = on ? (legacy ? h->s2_plan.ntz : h->res_plan.ntz) : 0;
   return on ? 1 : 0;
 }
 

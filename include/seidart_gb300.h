@@ -429,8 +429,9 @@ int32_t sfd_adjoint_gradient(sfd_handle* h, double* planes, int64_t count);
 
 /* ---- Batched runs ----------------------------------------------------------
  * Many 2-D models (electromag2 shots, seismic2 models of any sizes, mixed)
- * advance together in one persistent cooperative kernel launch with a grid
- * barrier per time step.  Replaces the per-shot process loop of the driver
+ * advance by one call.  Models that are faster alone on chip run so, one
+ * after another; the others advance together in one persistent cooperative
+ * kernel launch with a grid barrier per time step.  Replaces the per-shot process loop of the driver
  * (src/seidart/simulations/common_offset.py:143-284, one seidartfdtd call per
  * source).  The handles must be single-pass 2-D handles on one stream with
  * model and CPML set; each keeps its own state, source, receivers and traces.

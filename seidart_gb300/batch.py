@@ -3,8 +3,10 @@
 The reference runs one ``seidartfdtd`` process per source position and
 re-reads every snapshot afterwards (``src/seidart/simulations/common_offset.py:143-284``).
 Here every shot/model is an :class:`~seidart_gb300.solver.FDTDSolver` and a
-:class:`Batch` advances all of them together in one cooperative kernel launch
-per run (``sfd_batch_run``), with per-model receivers gathered on the device.
+:class:`Batch` advances all of them by one call (``sfd_batch_run``), with
+per-model receivers gathered on the device: models that are faster alone on
+chip run so, one after another, the others together in one cooperative kernel
+launch.
 
 :func:`autotune` picks the tile depth (rows per thread) and blocks per SM of
 that launch by timing a few steps of each candidate on the batch itself, and

@@ -169,6 +169,9 @@ void count_hand_overs(sfd_handle_s* h, int hand_overs);
 void reduce_norms(sfd_handle_s* h);
 // Whether this handle's runs go on chip (decided once per handle).
 bool resident_usable(sfd_handle_s* h);
+// The next nsteps steps of a handle whose runs go on chip, in one launch;
+// waits between its tiles give up after limit_ns.
+int run_on_chip(sfd_handle_s* h, int64_t nsteps, unsigned long long limit_ns);
 // The on-chip electromag2 and seismic2 runs of nsteps steps from the handle's state.
 Em2Resident resident_args(const sfd_handle_s* h, int64_t nsteps);
 Seis2Resident seis2_resident_args(const sfd_handle_s* h, int64_t nsteps);

@@ -637,6 +637,29 @@ Seis2Resident seis2_resident_args(const sfd_handle* h, int64_t nsteps) {
   return r;
 }
 
+int run_on_chip(sfd_handle* h, int64_t nsteps, unsigned long long limit_ns) {
+  const Layout& L = h->L;
+  if (h->cfg.kind == SFD_ELECTROMAG2) {
+    begin_run(h, h->step, em2_hand_overs((int)nsteps));
+    Em2Resident r = resident_args(h, nsteps);
+    r.limit_ns = limit_ns;
+    CK(em2_resident_launch(r, h->stream));
+  } else {
+    const bool legacy = legacy_quirks(h->cfg);
+    begin_run(h, h->step, legacy ? 0 : s2_hand_overs((int)nsteps));
+    // tags from an earlier run must not match: clear every edge word
+    if (legacy)
+      CK(cudaMemsetAsync(h->base + L.off_res, 0, res_scratch_bytes(L.P, L.NZ, res_edge_fields(h->cfg.kind)), h->stream));
+    Seis2Resident r = seis2_resident_args(h, nsteps);
+    r.limit_ns = limit_ns;
+    CK(legacy ? seis2_legacy_launch(r, h->stream) : seis2_resident_launch(r, h->stream));
+  }
+  reduce_norms(h);
+  CK(cudaGetLastError());
+  h->step += nsteps;
+  return SFD_OK;
+}
+
 int ensure_graph(sfd_handle* h, int p) {
   if (h->graph[p]) return SFD_OK;
   cudaGraph_t g = nullptr;
@@ -1538,23 +1561,8 @@ int32_t sfd_run(sfd_handle* h, int64_t nsteps) {
   const Layout& L = h->L;
   Ctl* ctl = (Ctl*)(h->base + L.off_ctl);
   float* slots = (float*)(h->base + L.off_slots);
-  const bool on_chip = resident_usable(h), em2 = h->cfg.kind == SFD_ELECTROMAG2;
-  begin_run(h, h->step, !on_chip ? 0 : em2 ? em2_hand_overs((int)nsteps) : s2_hand_overs((int)nsteps));
-  if (on_chip) {  // the whole run in one launch, state on chip
-    if (em2) {
-      CK(em2_resident_launch(resident_args(h, nsteps), h->stream));
-    } else if (legacy_quirks(h->cfg)) {
-      // tags from an earlier run must not match: clear every edge word
-      CK(cudaMemsetAsync(h->base + L.off_res, 0, res_scratch_bytes(L.P, L.NZ, res_edge_fields(h->cfg.kind)), h->stream));
-      CK(seis2_legacy_launch(seis2_resident_args(h, nsteps), h->stream));
-    } else {
-      CK(seis2_resident_launch(seis2_resident_args(h, nsteps), h->stream));
-    }
-    k_reduce_slots<<<1, 1024, 0, h->stream>>>(ctl, slots, L.nslots);
-    CK(cudaGetLastError());
-    h->step += nsteps;
-    return SFD_OK;
-  }
+  if (resident_usable(h)) return run_on_chip(h, nsteps, h->wait_ns);
+  begin_run(h, h->step);
   const int64_t chunks = h->cap_stream ? nsteps / kGraphSteps : 0;
   const int rem = (int)(nsteps - chunks * kGraphSteps);
   if (chunks > 0) {

@@ -1,5 +1,6 @@
-// C ABI, part 2: batched runs -- one persistent cooperative launch
-// (batch.cu) advancing many 2-D models, each with its own handle.
+// C ABI, part 2: batched runs of many 2-D models, each with its own handle:
+// the models that are faster so run on chip, one after another; the others in
+// one persistent cooperative launch (batch.cu).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -34,11 +35,46 @@ size_t batch_bytes(int n) {
          align256(sizeof(BatchGroup) * (size_t)n);
 }
 
+int run_together(sfd_batch_s* b, const std::vector<sfd_handle*>& models, int64_t nsteps);
+
 // Models that read the same coefficient planes and have the same geometry.
 bool same_group(const sfd_handle* a, const sfd_handle* b) {
   if (a->cfg.kind != b->cfg.kind || a->cfg.nx != b->cfg.nx || a->cfg.nz != b->cfg.nz) return false;
   if (a->cfg.kind == SFD_ELECTROMAG2) return a->em2s[0].CAx == b->em2s[0].CAx;
   return a->s2s[0].A11 == b->s2s[0].A11;
+}
+
+// Which models of a run of nsteps steps run on chip, each alone, one after
+// another; the others advance together in the persistent launch.  Times in us
+// measured on a GB300: a step of the persistent launch costs about 17 (its
+// grid barrier and the chain of its tiles), plus 6 for a million electromag2
+// cells and 18 for a million seismic2 cells; a model alone on chip 1.1 + 1.3
+// and 1.9 + 4 for a million cells, and 20 a run.  (Eight 1040 x 540 shots and
+// four elastic models of 126,000 to 185,000 cells took 107 a step in the
+// persistent launch and 24 one after another; 32 shots of 120 x 90 cells 23
+// and 34.)
+std::vector<char> choose_on_chip(const std::vector<sfd_handle*>& h, int64_t nsteps) {
+  const int n = (int)h.size();
+  std::vector<char> alone(n, 0), fits(n, 0);
+  double undecided_alone = 0.0, undecided_batch = 0.0, batch = 0.0;
+  auto cost = [&](int m, double* in_batch) {
+    const double cells = (double)h[m]->cfg.nx * h[m]->cfg.nz * 1e-6;
+    const bool em2 = h[m]->cfg.kind == SFD_ELECTROMAG2;
+    *in_batch = nsteps * cells * (em2 ? 6.0 : 18.0);
+    return 20.0 + nsteps * (em2 ? 1.1 + 1.3 * cells : (1.9 + 4.0 * cells) * (legacy_quirks(h[m]->cfg) ? 1.5 : 1.0));
+  };
+  for (int m = 0; m < n; ++m) {
+    double in_batch;
+    const double own = cost(m, &in_batch);
+    fits[m] = resident_usable(h[m]);
+    if (!fits[m]) batch += in_batch;
+    else if (own <= in_batch) alone[m] = 1;
+    else undecided_alone += own, undecided_batch += in_batch;
+  }
+  // the rest together: alone, unless the persistent launch runs anyway or is cheaper as a whole
+  if (batch == 0.0 && undecided_alone <= 17.0 * nsteps + undecided_batch)
+    for (int m = 0; m < n; ++m) alone[m] = fits[m];
+  return alone;
 }
 }  // namespace
 
@@ -101,6 +137,28 @@ int32_t sfd_batch_run(sfd_batch* b, int64_t nsteps) {
     if (b->h[m]->step + nsteps > b->h[m]->cfg.nstep)
       return fail(SFD_ERR_BAD_ARG, "model %d: run to step %lld exceeds its %d source samples", m,
                   (long long)(b->h[m]->step + nsteps), b->h[m]->cfg.nstep);
+  CK(cudaMemsetAsync(b->bar(), 0, sizeof(GridBarrier), b->stream));
+  std::vector<sfd_handle*> rest;  // the models of the persistent launch
+  const std::vector<char> alone = b->stall ? std::vector<char>(n, 0) : choose_on_chip(b->h, nsteps);
+  for (int m = 0; m < n; ++m) {
+    b->h[m]->adj_rec_n = 0;  // recorded states no longer follow from the handle
+    if (!alone[m]) {
+      rest.push_back(b->h[m]);
+      continue;
+    }
+    const int r = run_on_chip(b->h[m], nsteps, b->limit_ns);
+    if (r) return r;
+  }
+  return rest.empty() ? SFD_OK : run_together(b, rest, nsteps);
+}
+
+}  // extern "C"
+
+namespace {
+
+// nsteps steps of `models` in the persistent launch.
+int run_together(sfd_batch* b, const std::vector<sfd_handle*>& models, int64_t nsteps) {
+  const int n = (int)models.size();
   int maxb = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&maxb, batch_kernel_ptr(b->zb), 256, 0));
   const int bps = std::min(b->bps, maxb);
@@ -108,7 +166,7 @@ int32_t sfd_batch_run(sfd_batch* b, int64_t nsteps) {
   b->models.assign(n, BatchModel());
   b->steps.assign(n, 0);
   for (int m = 0; m < n; ++m) {
-    sfd_handle* h = b->h[m];
+    sfd_handle* h = models[m];
     BatchModel& md = b->models[m];
     md.kind = h->cfg.kind == SFD_ELECTROMAG2 ? SFD_BATCH_EM2 : SFD_BATCH_SEIS2;
     md.gx = md.kind == SFD_BATCH_EM2 ? (h->cfg.nx + 127) / 128 : (h->cfg.nx + 31) / 32;  // em2 tiles are 128 wide
@@ -126,7 +184,7 @@ int32_t sfd_batch_run(sfd_batch* b, int64_t nsteps) {
   int tile0 = 0;
   for (int m = 0; m < n;) {
     int e = m + 1;
-    while (e < n && same_group(b->h[m], b->h[e])) ++e;
+    while (e < n && same_group(models[m], models[e])) ++e;
     BatchGroup g;
     g.first = m;
     g.n = e - m;
@@ -147,12 +205,16 @@ int32_t sfd_batch_run(sfd_batch* b, int64_t nsteps) {
                   b->limit_ns, b->stall, b->stream));
   batch_end(b->dmodels(), n, (int)nsteps, b->stream);
   CK(cudaGetLastError());
-  for (sfd_handle* h : b->h) {
+  for (sfd_handle* h : models) {
     h->step += nsteps;
     h->cur ^= (int)(nsteps & 1);
   }
   return SFD_OK;
 }
+
+}  // namespace
+
+extern "C" {
 
 int32_t sfd_batch_set_wait_limit(sfd_batch* b, int64_t ns) {
   g_err.clear();

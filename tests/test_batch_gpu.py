@@ -100,3 +100,29 @@ def test_shared_model_batch_matches_separate_models(gpu):
         assert np.array_equal(a.traces(), b.traces())
     for s in own + shared:
         s.close()
+
+
+@pytest.mark.parametrize("tiny,large", [(36, 0), (2, 1)], ids=["many small", "one too large for the chip"])
+def test_persistent_launch(gpu, tiny, large):
+    """Batches that take the persistent launch: many models too small to fill
+    the chip alone, and small ones beside a model that does not fit on chip.
+    Handles that never run on chip (FLAG_STREAMING) go with them."""
+    cases = [sy.small_case(ELECTROMAG2 if q % 3 else SEISMIC2, seed=90 + q, nx=41 + 3 * (q % 7), nz=37 + 2 * (q % 5),
+                           npml=5, nstep=40) for q in range(tiny)]
+    cases += [sy.small_case(ELECTROMAG2, seed=200, nx=1300, nz=1100, npml=9, nstep=40)] * large
+    flags = [FLAG_STREAMING if q % 5 == 4 else 0 for q in range(len(cases))]
+    solvers = [make_solver(c, flags=f) for c, f in zip(cases, flags)]
+    b = Batch(solvers)
+    b.run(17)
+    b.run(23)
+    b.status()
+    for c, s in list(zip(cases, solvers))[-8:]:
+        with make_solver(c, flags=FLAG_STREAMING) as one:
+            one.run(c.nstep)
+            one.status()
+            assert rel_l2(s.traces(), one.traces()) <= 1e-6
+            for name in ("Ex", "Ez", "Hy") if c.grid.kind == ELECTROMAG2 else ("vx", "vz", "sigmaxz"):
+                assert rel_l2(s.field(name), one.field(name)) <= 1e-6, name
+    b.close()
+    for s in solvers:
+        s.close()

@@ -49,6 +49,14 @@ __device__ __forceinline__ void st_word(uint4* p, float x, float y, float z, uns
                "l"(b));
 }
 
+// Copies 16 bytes from global to shared memory without a register, or writes
+// zeros (on = false); the copying thread may read them after copies_wait.
+__device__ __forceinline__ void copy16(float* dst, const float* src, bool on) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(on ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // The larger of a and b, NaN if either is.
 __device__ __forceinline__ float max_nan(float a, float b) {
   float d;

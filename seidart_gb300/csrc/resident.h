@@ -134,8 +134,10 @@ struct ResDump {
 
 struct Em2Resident {
   int NX, NZ, P, W;
-  float *Ex, *Ez, *Hy;               // current copy: read before, written after the run
-  float *mExz, *mEzx, *mHyz, *mHyx;  // z-, x-, z-, x-strip memory variables of the current copy
+  float *Ex, *Ez, *Hy;               // the state before the run
+  float *mExz, *mEzx, *mHyz, *mHyx;  // its z-, x-, z-, x-strip memory variables
+  // where the state after it goes: the same arrays (on chip), the other copy (streaming)
+  float *oEx, *oEz, *oHy, *omExz, *omEzx, *omHyz, *omHyx;
   const float *CAx, *CBx, *CAz, *CBz;
   AxisTab X, Z;
   float dbH;
@@ -235,6 +237,14 @@ bool em2_resident_plan(int NX, int NZ, int npml, int max_ctas, size_t max_smem, 
 // CTAs of the plan fit on one SM.
 cudaError_t em2_resident_prepare(const TilePlan& plan, int* ctas_per_sm);
 cudaError_t em2_resident_launch(const Em2Resident& a, cudaStream_t s);
+// Streaming runs (em2_stream.cu): their tiles, and a launch of at most
+// kTileHalo steps (a.nsteps) from one copy of the state to the other.
+struct StreamPlan {
+  int ntx, nbz;
+  size_t smem;
+};
+cudaError_t em2_stream_prepare(int NX, int NZ, int W, StreamPlan* out);
+void em2_stream_launch(const Em2Resident& a, const StreamPlan& plan, cudaStream_t s);
 
 // The same for the adjoint sweep's tiles.
 bool em2_adj_resident_plan(int NX, int NZ, int npml, int max_ctas, size_t max_smem, ResPlan* out);

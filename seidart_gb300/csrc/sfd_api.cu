@@ -179,11 +179,11 @@ int choose_ysplit(const sfd_config& c) {
   return s;
 }
 
-// Whether the single-pass 2-D steps keep memory variable q in two copies
-// (those of the first half-step, re-derived on tile halos).
+// Whether the single-pass 2-D steps keep memory variable q in two copies:
+// those that are re-derived on tile halos.
 bool pingpong_mem(int kind, int q) {
   switch (kind) {
-    case SFD_ELECTROMAG2: return q < 2;                // dEx_dz dEz_dx
+    case SFD_ELECTROMAG2: return q < 4;
     case SFD_SEISMIC2: return q < 4 || (q >= 8 && q < 12);  // the velocity-gradient ones of both stress loops
   }
   return false;
@@ -346,8 +346,8 @@ bool bind_args(sfd_handle* h) {
         b.mExz0 = h->mc(0, p); b.mEzx0 = h->mc(1, p);
         b.Ex1 = h->fc(0, 1 - p); b.Ez1 = h->fc(1, 1 - p); b.Hy1 = h->fc(2, 1 - p);
         b.mExz1 = h->mc(0, 1 - p); b.mEzx1 = h->mc(1, 1 - p);
-        b.mHyz = h->mc(2, 0); b.mHyx = h->mc(3, 0);
-        b.mHyz0 = b.mHyz; b.mHyx0 = b.mHyx;
+        b.mHyz0 = h->mc(2, p); b.mHyx0 = h->mc(3, p);
+        b.mHyz = h->mc(2, 1 - p); b.mHyx = h->mc(3, 1 - p);
         b.CAx = a.CAx; b.CBx = a.CBx; b.CAz = a.CAz; b.CBz = a.CBz;
         b.X = a.X; b.Z = a.Z; b.dbH = a.dbH; b.io = io;
       }
@@ -592,7 +592,9 @@ Em2Resident resident_args(const sfd_handle* h, int64_t nsteps) {
   const Em2Step& b = h->em2s[h->cur];
   r.NX = b.NX; r.NZ = b.NZ; r.P = b.P; r.W = b.W;
   r.Ex = h->fc(0, h->cur); r.Ez = h->fc(1, h->cur); r.Hy = h->fc(2, h->cur);
-  r.mExz = h->mc(0, h->cur); r.mEzx = h->mc(1, h->cur); r.mHyz = h->mc(2, 0); r.mHyx = h->mc(3, 0);
+  r.mExz = h->mc(0, h->cur); r.mEzx = h->mc(1, h->cur); r.mHyz = h->mc(2, h->cur); r.mHyx = h->mc(3, h->cur);
+  r.oEx = r.Ex; r.oEz = r.Ez; r.oHy = r.Hy;
+  r.omExz = r.mExz; r.omEzx = r.mEzx; r.omHyz = r.mHyz; r.omHyx = r.mHyx;
   r.CAx = b.CAx; r.CBx = b.CBx; r.CAz = b.CAz; r.CBz = b.CBz;
   r.X = b.X; r.Z = b.Z; r.dbH = b.dbH;
   r.io = b.io;
@@ -658,6 +660,14 @@ int run_on_chip(sfd_handle* h, int64_t nsteps, unsigned long long limit_ns) {
   CK(cudaGetLastError());
   h->step += nsteps;
   return SFD_OK;
+}
+
+// Launches of a streaming run that advances up to `most` steps a launch, from
+// copy to copy of the state: of the steps' parity, so that the state after the
+// run lies in the copy that one launch a step would leave it in.
+int64_t stream_launches(int64_t nsteps, int64_t most) {
+  const int64_t n = (nsteps + most - 1) / most;
+  return n + ((n ^ nsteps) & 1);
 }
 
 int ensure_graph(sfd_handle* h, int p) {
@@ -1563,6 +1573,25 @@ int32_t sfd_run(sfd_handle* h, int64_t nsteps) {
   float* slots = (float*)(h->base + L.off_slots);
   if (resident_usable(h)) return run_on_chip(h, nsteps, h->wait_ns);
   begin_run(h, h->step);
+  if (h->single && h->cfg.kind == SFD_ELECTROMAG2) {
+    StreamPlan plan;
+    CK(em2_stream_prepare(h->cfg.nx, h->cfg.nz, h->cfg.npml, &plan));
+    const int64_t n = stream_launches(nsteps, kTileHalo);
+    for (int64_t l = 0; l < n; ++l) {
+      const int64_t s0 = nsteps * l / n, s1 = nsteps * (l + 1) / n;
+      Em2Resident r = resident_args(h, s1 - s0);
+      const int q = 1 - h->cur;
+      r.oEx = h->fc(0, q); r.oEz = h->fc(1, q); r.oHy = h->fc(2, q);
+      r.omExz = h->mc(0, q); r.omEzx = h->mc(1, q); r.omHyz = h->mc(2, q); r.omHyx = h->mc(3, q);
+      r.t0 += (int)s0;
+      em2_stream_launch(r, plan, h->stream);
+      h->cur = q;
+    }
+    reduce_norms(h);
+    CK(cudaGetLastError());
+    h->step += nsteps;
+    return SFD_OK;
+  }
   const int64_t chunks = h->cap_stream ? nsteps / kGraphSteps : 0;
   const int rem = (int)(nsteps - chunks * kGraphSteps);
   if (chunks > 0) {

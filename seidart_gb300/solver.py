@@ -113,8 +113,8 @@ class FDTDSolver:
 
     ``flags`` = ``FLAG_TWO_PASS`` selects, for the 2-D kinds, the two-kernel
     step (fields updated in place) instead of the default single-pass step.
-    ``FLAG_STREAMING`` keeps one launch per step even where the grid would
-    fit on chip (by default an electromag2 grid that fits in the SMs' shared
+    ``FLAG_STREAMING`` streams the state through device memory even where it would
+    fit on chip (by default a 2-D grid that fits in the SMs' shared
     memory runs a whole ``run`` in one launch with the state held on chip).
 
     ``nstep`` is the number of source samples (the run length); ``nrec`` the
@@ -301,7 +301,7 @@ class FDTDSolver:
 
     def on_chip(self):
         """(tiles, tile rows) when ``run`` keeps the whole state on chip (one
-        launch per run, one CTA per tile), else None (one launch per step)."""
+        launch per run, one CTA per tile), else None (streaming launches)."""
         tx, tz = C.c_int32(), C.c_int32()
         rc = self._L.sfd_on_chip(self._h, C.byref(tx), C.byref(tz))
         if rc < 0:

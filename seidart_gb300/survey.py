@@ -129,7 +129,7 @@ def gpu_runner(cases, device=None, schedule: str = "sequential") -> List[np.ndar
 
     * ``"sequential"`` (default): every case alone, one after another, each
       in its own default form -- the whole run in one launch on chip where
-      the grid fits, else one launch per step -- through a
+      the grid fits, else streaming -- through a
       :class:`~seidart_gb300.solver.ShotPipeline` (two handles in turn, a
       case's host work overlapping the previous case's run);
     * ``"batch"``: all of them advancing together in one persistent launch

@@ -2,8 +2,8 @@
 // scheme of electromag2 with complex permittivities, hence complex update
 // coefficients, fields and CPML memory variables.  Complex arrays are held
 // as separate real and imaginary planes (x fastest, pitch P), so each plane
-// streams like a real field.  Two kernels per step, as the two-pass
-// electromag2 (em2.cu):
+// streams like a real field.  Two kernels per step (SFD_FLAG_TWO_PASS; other
+// runs: em2c_stream.cu), as the two-pass electromag2 (em2.cu):
 //   half1: Hy (:530-549) with the dEx/dz, dEz/dx memory variables; block
 //          (0,0) first records the receivers of the previous step;
 //   half2: Ex (:556-565), Ez (:567-576) with the dHy memory variables, the

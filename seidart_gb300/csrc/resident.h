@@ -240,11 +240,22 @@ cudaError_t em2_resident_launch(const Em2Resident& a, cudaStream_t s);
 // Streaming runs (em2_stream.cu): their tiles, and a launch of at most
 // kTileHalo steps (a.nsteps) from one copy of the state to the other.
 struct StreamPlan {
-  int ntx, nbz;
+  int ntx, nbz, rb;  // rb: rows a warp (electromag2c)
   size_t smem;
 };
 cudaError_t em2_stream_prepare(int NX, int NZ, int W, StreamPlan* out);
 void em2_stream_launch(const Em2Resident& a, const StreamPlan& plan, cudaStream_t s);
+
+// Streaming electromag2c runs (em2c_stream.cu): at most kC2Halo steps a launch
+// from one copy of the state (`from`) to the other.
+constexpr int kC2Halo = 4;
+struct Em2cStream {
+  Em2cArgs from;
+  float *Ex[2], *Ez[2], *Hy[2], *mExz[2], *mEzx[2], *mHyz[2], *mHyx[2];
+  int t0, nsteps;
+};
+cudaError_t em2c_stream_prepare(int NX, int NZ, int W, StreamPlan* out);
+void em2c_stream_launch(const Em2cStream& a, const StreamPlan& plan, cudaStream_t s);
 
 // The same for the adjoint sweep's tiles.
 bool em2_adj_resident_plan(int NX, int NZ, int npml, int max_ctas, size_t max_smem, ResPlan* out);

@@ -184,6 +184,7 @@ int choose_ysplit(const sfd_config& c) {
 bool pingpong_mem(int kind, int q) {
   switch (kind) {
     case SFD_ELECTROMAG2: return q < 4;
+    case SFD_ELECTROMAG2C: return q < 8;
     case SFD_SEISMIC2: return q < 4 || (q >= 8 && q < 12);  // the velocity-gradient ones of both stress loops
   }
   return false;
@@ -195,6 +196,11 @@ bool legacy_quirks(const sfd_config& c) { return (c.flags & SFD_FLAG_LEGACY_QUIR
 bool single_pass(const sfd_config& c) {
   return has_single_pass(c.kind) && !(c.flags & (SFD_FLAG_TWO_PASS | SFD_FLAG_CPML_2D));
 }
+
+// Whether a handle's runs stream from one copy of the state to the other and
+// back (electromag2c: an even number of launches, so that a state between
+// runs lies in the first copy).
+bool streams_complex(const sfd_config& c) { return c.kind == SFD_ELECTROMAG2C && !(c.flags & SFD_FLAG_TWO_PASS); }
 
 // Edge fields of an on-chip run (resident.h): electromag2 2, seismic2 6.
 int res_edge_fields(int kind) { return kind == SFD_SEISMIC2 ? 6 : 2; }
@@ -255,7 +261,7 @@ void make_layout(const sfd_config& c, Layout* L) {
   }
   L->off_fieldsB = 0;
   for (int m = 0; m < 18; ++m) L->off_memB[m] = 0;
-  if (single_pass(c)) {
+  if (single_pass(c) || streams_complex(c)) {
     L->off_fieldsB = o; o += align256(sizeof(float) * L->fsz * nfields(c.kind));
     for (int m = 0; m < nm; ++m)
       if (pingpong_mem(c.kind, m)) { L->off_memB[m] = o; o += align256(sizeof(float) * L->mem_sz[m]); }
@@ -1586,6 +1592,31 @@ int32_t sfd_run(sfd_handle* h, int64_t nsteps) {
       r.t0 += (int)s0;
       em2_stream_launch(r, plan, h->stream);
       h->cur = q;
+    }
+    reduce_norms(h);
+    CK(cudaGetLastError());
+    h->step += nsteps;
+    return SFD_OK;
+  }
+  if (streams_complex(h->cfg)) {
+    StreamPlan plan;
+    CK(em2c_stream_prepare(h->cfg.nx, h->cfg.nz, h->cfg.npml, &plan));
+    const int64_t pairs = (nsteps + 2 * kC2Halo - 1) / (2 * kC2Halo), n = 2 * pairs;
+    Em2cStream r;
+    r.from = h->em2c;
+    for (int64_t l = 0; l < n; ++l) {
+      const int from = (int)(l & 1), to = 1 - from;
+      for (int q = 0; q < 2; ++q) {
+        r.from.Ex[q] = h->fc(q, from); r.from.Ez[q] = h->fc(2 + q, from); r.from.Hy[q] = h->fc(4 + q, from);
+        r.from.mExz[q] = h->mc(q, from); r.from.mEzx[q] = h->mc(2 + q, from);
+        r.from.mHyz[q] = h->mc(4 + q, from); r.from.mHyx[q] = h->mc(6 + q, from);
+        r.Ex[q] = h->fc(q, to); r.Ez[q] = h->fc(2 + q, to); r.Hy[q] = h->fc(4 + q, to);
+        r.mExz[q] = h->mc(q, to); r.mEzx[q] = h->mc(2 + q, to); r.mHyz[q] = h->mc(4 + q, to); r.mHyx[q] = h->mc(6 + q, to);
+      }
+      const int64_t s0 = nsteps * l / n, s1 = nsteps * (l + 1) / n;
+      r.t0 = (int)(h->step + s0);
+      r.nsteps = (int)(s1 - s0);
+      em2c_stream_launch(r, plan, h->stream);
     }
     reduce_norms(h);
     CK(cudaGetLastError());

@@ -166,11 +166,10 @@ class TraceModel(_Checkpointed):
                          record=record)
 
     def planes_for(self, eps11, eps33, sigma):
-        p = self.base.copy()
-        p[0] = np.asarray(eps11, dtype=np.float64)
-        p[2] = np.asarray(eps33, dtype=np.float64)
-        p[3] = np.asarray(sigma, dtype=np.float64)
-        p[5] = np.asarray(sigma, dtype=np.float64)
+        p = np.empty_like(self.base)
+        p[0], p[1], p[2] = eps11, self.base[1], eps33  # converted as they are written
+        p[3], p[4] = sigma, self.base[4]
+        p[5] = p[3]
         return p
 
     def forward(self, eps11, eps33, sigma):

@@ -26,6 +26,8 @@
 namespace sfd {
 
 using namespace res;
+using tile2::copies_wait;
+using tile2::copy8;
 using tile2::max_nan;
 
 namespace {
@@ -51,11 +53,6 @@ __device__ __forceinline__ float el(const float2& v, int e) { return (&v.x)[e]; 
 __device__ __forceinline__ float2& part(cf2& v, int q) { return q ? v.i : v.r; }
 __device__ __forceinline__ float2 lds(int o) { return *reinterpret_cast<const float2*>(c2_smem + o); }
 __device__ __forceinline__ void sts(int o, float2 v) { *reinterpret_cast<float2*>(c2_smem + o) = v; }
-__device__ __forceinline__ void copy8(float* dst, const float* src, bool on) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(on ? 8 : 0) : "memory");
-}
-
 // Tiles of uniform size: ntx columns of at most 56 cells (one of up to 64), nbz
 // bands of at most kWarps RB - 2 kC2Halo rows (one of up to kWarps RB).
 __host__ __device__ inline int cut_x(int NX, int c, int ntx) {
@@ -237,7 +234,7 @@ __device__ __forceinline__ void em2c_tile(const Em2cStream& a, C2Tile& G, const 
   __syncthreads();
   const bool listed = G.nrec <= kMaxRec;
   const int rec0 = listed ? G.first[tid] : own ? 0 : -1;  // this thread's first receiver; not listed: all are looked at
-  if (CS) asm volatile("cp.async.wait_all;" ::: "memory");  // each thread reads only what it copied
+  if (CS) copies_wait();  // each thread reads only what it copied
   if (CS && EDGE) {  // loop bounds and planes into the coefficients: (1, 0) carries a cell over, (0, 0) holds it at zero
 #pragma unroll 1
     for (int j = 0; j < nr; ++j) {

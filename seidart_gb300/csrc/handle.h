@@ -65,7 +65,7 @@ int res_edge_fields(int kind);
 struct Layout {
   int P, NX, NY, NZ, W, ysplit, nslots;
   size_t fsz;  // floats per field
-  size_t off_ctl, off_fields, off_mem[18], mem_sz[18], off_fieldsB, off_memB[18], off_coef, coef_plane, off_axis[3],
+  size_t off_ctl, off_fields, off_mem[18], mem_sz[18], off_fieldsB, off_memB[18], off_memS[4], off_coef, coef_plane, off_axis[3],
       off_q3, off_src, off_rec, off_traces, off_slots, off_res, off_words, total;
 };
 

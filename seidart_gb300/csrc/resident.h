@@ -217,6 +217,7 @@ struct Seis2Resident {
   unsigned long long limit_ns;
   unsigned tag_bias;  // added to every awaited edge tag; 0 except in the timeout test aid
   S2Dump dump;        // base != nullptr: dump every step's state, leave the loaded state as it was
+  float* out[17];     // streaming: where the state after the run goes, in S2Dump's order
 };
 
 // Tiling of an NX x NZ seismic2 grid for `max_ctas` CTAs of at most
@@ -240,11 +241,15 @@ cudaError_t em2_resident_launch(const Em2Resident& a, cudaStream_t s);
 // Streaming runs (em2_stream.cu): their tiles, and a launch of at most
 // kTileHalo steps (a.nsteps) from one copy of the state to the other.
 struct StreamPlan {
-  int ntx, nbz, rb;  // rb: rows a warp (electromag2c)
+  int ntx, nbz, rb;  // rb: rows a warp (electromag2c, seismic2)
   size_t smem;
 };
 cudaError_t em2_stream_prepare(int NX, int NZ, int W, StreamPlan* out);
 void em2_stream_launch(const Em2Resident& a, const StreamPlan& plan, cudaStream_t s);
+
+// The same for seismic2 (s2_stream.cu), at most kS2Steps steps a launch.
+cudaError_t seis2_stream_prepare(int NX, int NZ, int W, StreamPlan* out);
+void seis2_stream_launch(const Seis2Resident& a, const StreamPlan& plan, cudaStream_t s);
 
 // Streaming electromag2c runs (em2c_stream.cu): at most kC2Halo steps a launch
 // from one copy of the state (`from`) to the other.

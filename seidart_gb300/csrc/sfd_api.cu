@@ -202,6 +202,10 @@ bool single_pass(const sfd_config& c) {
 // runs lies in the first copy).
 bool streams_complex(const sfd_config& c) { return c.kind == SFD_ELECTROMAG2C && !(c.flags & SFD_FLAG_TWO_PASS); }
 
+// The same for seismic2 with the corrected physics (each run starts and ends in
+// the copy that holds the state).
+bool streams_seis2(const sfd_config& c) { return c.kind == SFD_SEISMIC2 && single_pass(c) && !legacy_quirks(c); }
+
 // Edge fields of an on-chip run (resident.h): electromag2 2, seismic2 6.
 int res_edge_fields(int kind) { return kind == SFD_SEISMIC2 ? 6 : 2; }
 
@@ -266,6 +270,11 @@ void make_layout(const sfd_config& c, Layout* L) {
     for (int m = 0; m < nm; ++m)
       if (pingpong_mem(c.kind, m)) { L->off_memB[m] = o; o += align256(sizeof(float) * L->mem_sz[m]); }
   }
+  // a streaming seismic2 run's other copy of the stress-gradient variables,
+  // which the single-pass step updates in place
+  for (int m = 0; m < 4; ++m) L->off_memS[m] = 0;
+  if (streams_seis2(c))
+    for (int m = 0; m < 4; ++m) { L->off_memS[m] = o; o += align256(sizeof(float) * L->mem_sz[4 + m]); }
   L->coef_plane = (size_t)L->P * c.nz;
   // the update coefficients, then (2-D CPML fields) 1/K, a, b of the full and half offsets
   L->off_coef = o; o += align256(sizeof(float) * L->coef_plane * (ncoef(c.kind) + (cpml2d(c) ? 6 : 0)));
@@ -1564,6 +1573,29 @@ int32_t sfd_run(sfd_handle* h, int64_t nsteps) {
       r.t0 += (int)s0;
       em2_stream_launch(r, plan, h->stream);
       h->cur = q;
+    }
+    reduce_norms(h);
+    CK(cudaGetLastError());
+    h->step += nsteps;
+    return SFD_OK;
+  }
+  if (streams_seis2(h->cfg)) {
+    StreamPlan plan;
+    CK(seis2_stream_prepare(h->cfg.nx, h->cfg.nz, h->cfg.npml, &plan));
+    const int64_t n = 2 * ((nsteps + 2 * kS2Steps - 1) / (2 * kS2Steps));
+    Seis2Resident r = seis2_resident_args(h, 0);
+    float** at[17] = {&r.vx, &r.vz, &r.sxx, &r.szz, &r.sxz, &r.m_vxx, &r.m_vzz, &r.m_vxz, &r.m_vzx, &r.m_sxx_x, &r.m_szz_z,
+                      &r.m_sxz_x, &r.m_sxz_z, &r.m2_vxx, &r.m2_vzz, &r.m2_vxz, &r.m2_vzx};
+    for (int q = 0; q < 17; ++q)
+      r.out[q] = q < 5             ? h->fc(q, 1 - h->cur)
+                 : q < 9 || q > 12 ? h->mc(q - 5, 1 - h->cur)
+                                   : (float*)(h->base + L.off_memS[q - 9]);
+    for (int64_t l = 0; l < n; ++l) {
+      const int64_t s0 = nsteps * l / n, s1 = nsteps * (l + 1) / n;
+      r.t0 = (int)(h->step + s0);
+      r.nsteps = (int)(s1 - s0);
+      seis2_stream_launch(r, plan, h->stream);
+      for (int q = 0; q < 17; ++q) std::swap(*at[q], r.out[q]);
     }
     reduce_norms(h);
     CK(cudaGetLastError());

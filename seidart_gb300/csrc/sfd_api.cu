@@ -553,7 +553,7 @@ bool resident_usable(sfd_handle* h) {
   const size_t smem = (size_t)optin - static_smem;
   const sfd_config& c = h->cfg;
   int per_sm = 0;
-  bool fits;  // the tilings are searched in tens of microseconds, not cached
+  bool fits;  // the tilings are searched in 0.02 to 0.2 ms, not cached
   if (legacy_quirks(c))
     fits = seis2_legacy_plan(c.nx, c.nz, ctas, smem, &h->s2_plan) && seis2_legacy_prepare(h->s2_plan, &per_sm) == cudaSuccess;
   else if (c.kind == SFD_SEISMIC2)

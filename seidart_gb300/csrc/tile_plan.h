@@ -64,12 +64,13 @@ bool plan_tiles(const TileRules& t, int NX, int NZ, int W, int max_ctas, size_t 
     int n = 0, z = 0;
     if (cuts) cuts->assign(1, 0);
     while (z < NZ) {
-      int z1 = z;
-      while (z1 < NZ) {
-        const Frame f = frame(c, z, z1 + 1);
+      // the deepest band that fits, by bisection: rows, cost and memory grow with it
+      int z1 = z, over = std::min(NZ, z + max_rows) + 1;
+      while (over - z1 > 1) {
+        const int m = (z1 + over) / 2;
+        const Frame f = frame(c, z, m);
         const double cost = (f.rows + t.zrow * (f.zlo + f.zhi)) * (f.xlanes ? 1.0 + t.xcol : 1.0);
-        if (cost > C || f.rows > max_rows || smem(f, t.max_rb) > max_smem) break;
-        ++z1;
+        (cost > C || f.rows > max_rows || smem(f, t.max_rb) > max_smem ? over : z1) = m;
       }
       if (z1 == z) return max_ctas + 1;
       // a last band of a few rows: no thinner than its neighbours' halo

@@ -67,9 +67,10 @@ extern "C" {
 /* Flags (sfd_config.flags). */
 #define SFD_FLAG_TWO_PASS 1 /* 2-D kinds: two kernels per step (one per half-step,
                                fields updated in place) instead of the default
-                               single-pass step over ping-pong copies */
-#define SFD_FLAG_STREAMING 2 /* 2-D single-pass kinds: one launch per step even
-                               when the grid fits on chip (by default a run of
+                               steps over two copies of the state */
+#define SFD_FLAG_STREAMING 2 /* 2-D single-pass kinds: the state streams through
+                               device memory, a few steps a launch, even when the
+                               grid fits on chip (by default a run of
                                a grid that fits in the SMs' shared memory is
                                one launch with the state held on chip) */
 /* Seismic kinds: reproduce the legacy Fortran loops' quirks instead of the
@@ -328,7 +329,7 @@ int32_t sfd_field_device(const sfd_handle* h, int32_t field, float** ptr, int64_
 int32_t sfd_launch_half(sfd_handle* h, int32_t which, int32_t count);
 
 /* Whether sfd_run keeps this handle's whole state on chip (one launch per run,
- * one CTA per tile of the grid): 1 yes, 0 no (one launch per step).  Single-
+ * one CTA per tile of the grid): 1 yes, 0 no (a few steps a launch).  Single-
  * pass electromag2 and seismic2 handles whose grid fits the SMs' shared
  * memory (and registers) run on chip; decided on the current device from its
  * SM count and shared memory.  tiles and

@@ -383,7 +383,7 @@ def bench_batched(device, flush, stream, peak, plain_value, runs=2, nstep=4000, 
            "value": round(value, 3), "unit": METRIC, "ms_per_run": round(ms, 2), "cells": cells,
            "bytes_per_cell_update": round(step_bytes / cells, 2),
            "bytes_per_cell_update_unshared": round(unshared / cells, 2),
-           "roofline": {"bound": "hbm", "kernel": "batch_kernel", "achieved": round(achieved, 1), "peak": peak,
+           "roofline": {"bound": "hbm", "kernel": "em2_resident_kernel, seis2_resident_kernel, batch_kernel", "achieved": round(achieved, 1), "peak": peak,
                         "unit": "GB/s", "frac": round(achieved / peak, 4)},
            "vs_plain_single_shot": round(value / plain_value, 3) if plain_value else None,
            "plain_sequential": {"value": round(plain_agg, 3), "unit": METRIC, "ms_per_run": round(plain_ms, 2),

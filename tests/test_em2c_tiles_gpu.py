@@ -1,8 +1,8 @@
 """GPU: electromag2c runs at the sizes where the streaming tiles change, against
 the FP64 oracle: widths around one column of tiles (64 cells) and two (112),
-depths around one band (40 rows) and around its cuts (32 owned rows), strips
-deeper than a tile, and pieces that are no multiple of the steps a launch
-advances.  Tolerances as in test_complex_em_gpu.py."""
+strips deeper than a tile, pieces that are no multiple of the steps a launch
+advances, grids whose tiles have one to five rows a warp, and strips that leave
+a tile's coefficients no room on chip.  Tolerances as in test_complex_em_gpu.py."""
 import numpy as np
 import pytest
 
@@ -30,10 +30,18 @@ def check(s, st, ref):
     (90, 131, 33, (64, 99)),
     (7, 6, 1, (3, 14)),
     (230, 73, 12, (150, 3)),
+    (400, 170, 10, (9, 30)),    # two rows a warp
+    (601, 400, 20, (17, 20)),   # three
+    (900, 440, 15, (20, 5)),    # four
+    (1040, 540, 20, (9, 20)),   # five
+    (1039, 539, 60, (10, 19)),  # five, coefficients read from L2 in the corners
 ])
 def test_tile_edges(gpu, nx, nz, npml, chunks):
     case = sy.small_case(ELECTROMAG2C, seed=nx + nz, nx=nx, nz=nz, npml=npml, nstep=sum(chunks), nrec=40)
     case.rec_ijk[:4] = [(nx - 1, 0, nz // 2), (nx - 2, 0, nz - 2), (0, 0, 0), (nx // 2, 0, nz - 1)]
+    if nx > 300:  # a few steps: from a corner, so that the strips see the wave
+        case.src_ijk = (nx - npml - 5, 0, nz - npml - 4)
+        case.rec_ijk[4:] = [(nx - npml - 30 + q, 0, nz - npml - 10 + q % 7) for q in range(36)]
     st, ref, _, blew = run_oracle(case)
     assert not blew
     with make_solver(case) as s:

@@ -197,13 +197,12 @@ bool single_pass(const sfd_config& c) {
   return has_single_pass(c.kind) && !(c.flags & (SFD_FLAG_TWO_PASS | SFD_FLAG_CPML_2D));
 }
 
-// Whether a handle's runs stream from one copy of the state to the other and
-// back (electromag2c: an even number of launches, so that a state between
-// runs lies in the first copy).
+// Whether a handle's runs stream from one copy of the state to the other
+// (electromag2c: a state between runs lies in the first copy).
 bool streams_complex(const sfd_config& c) { return c.kind == SFD_ELECTROMAG2C && !(c.flags & SFD_FLAG_TWO_PASS); }
 
-// The same for seismic2 with the corrected physics (each run starts and ends in
-// the copy that holds the state).
+// The same for seismic2 with the corrected physics (the copy that one launch a
+// step would leave a state in holds it).
 bool streams_seis2(const sfd_config& c) { return c.kind == SFD_SEISMIC2 && single_pass(c) && !legacy_quirks(c); }
 
 // Edge fields of an on-chip run (resident.h): electromag2 2, seismic2 6.
@@ -1582,7 +1581,7 @@ int32_t sfd_run(sfd_handle* h, int64_t nsteps) {
   if (streams_seis2(h->cfg)) {
     StreamPlan plan;
     CK(seis2_stream_prepare(h->cfg.nx, h->cfg.nz, h->cfg.npml, &plan));
-    const int64_t n = 2 * ((nsteps + 2 * kS2Steps - 1) / (2 * kS2Steps));
+    const int64_t n = stream_launches(nsteps, kS2Steps);
     Seis2Resident r = seis2_resident_args(h, 0);
     float** at[17] = {&r.vx, &r.vz, &r.sxx, &r.szz, &r.sxz, &r.m_vxx, &r.m_vzz, &r.m_vxz, &r.m_vzx, &r.m_sxx_x, &r.m_szz_z,
                       &r.m_sxz_x, &r.m_sxz_z, &r.m2_vxx, &r.m2_vzz, &r.m2_vxz, &r.m2_vzx};
@@ -1596,7 +1595,11 @@ int32_t sfd_run(sfd_handle* h, int64_t nsteps) {
       r.nsteps = (int)(s1 - s0);
       seis2_stream_launch(r, plan, h->stream);
       for (int q = 0; q < 17; ++q) std::swap(*at[q], r.out[q]);
+      h->cur ^= 1;
     }
+    for (int m = 0; m < 4 && (n & 1); ++m)  // the in-place variables have one copy that stays
+      CK(cudaMemcpyAsync(h->mc(4 + m, 0), h->base + L.off_memS[m], sizeof(float) * L.mem_sz[4 + m],
+                         cudaMemcpyDeviceToDevice, h->stream));
     reduce_norms(h);
     CK(cudaGetLastError());
     h->step += nsteps;
@@ -1605,7 +1608,7 @@ int32_t sfd_run(sfd_handle* h, int64_t nsteps) {
   if (streams_complex(h->cfg)) {
     StreamPlan plan;
     CK(em2c_stream_prepare(h->cfg.nx, h->cfg.nz, h->cfg.npml, &plan));
-    const int64_t pairs = (nsteps + 2 * kC2Halo - 1) / (2 * kC2Halo), n = 2 * pairs;
+    const int64_t n = (nsteps + kC2Halo - 1) / kC2Halo;
     Em2cStream r;
     r.from = h->em2c;
     for (int64_t l = 0; l < n; ++l) {
@@ -1621,6 +1624,11 @@ int32_t sfd_run(sfd_handle* h, int64_t nsteps) {
       r.t0 = (int)(h->step + s0);
       r.nsteps = (int)(s1 - s0);
       em2c_stream_launch(r, plan, h->stream);
+    }
+    if (n & 1) {  // back to the first copy: its fields and its memory variables lie back to back, the second's likewise
+      CK(cudaMemcpyAsync(h->fc(0, 0), h->fc(0, 1), sizeof(float) * L.fsz * 6, cudaMemcpyDeviceToDevice, h->stream));
+      CK(cudaMemcpyAsync(h->mc(0, 0), h->mc(0, 1), L.off_memB[7] - L.off_memB[0] + sizeof(float) * L.mem_sz[7],
+                         cudaMemcpyDeviceToDevice, h->stream));
     }
     reduce_norms(h);
     CK(cudaGetLastError());

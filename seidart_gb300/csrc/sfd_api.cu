@@ -1581,7 +1581,7 @@ int32_t sfd_run(sfd_handle* h, int64_t nsteps) {
   if (streams_seis2(h->cfg)) {
     StreamPlan plan;
     CK(seis2_stream_prepare(h->cfg.nx, h->cfg.nz, h->cfg.npml, &plan));
-    const int64_t n = stream_launches(nsteps, kS2Steps);
+    const int64_t n = (nsteps + kS2Steps - 1) / kS2Steps;
     Seis2Resident r = seis2_resident_args(h, 0);
     float** at[17] = {&r.vx, &r.vz, &r.sxx, &r.szz, &r.sxz, &r.m_vxx, &r.m_vzz, &r.m_vxz, &r.m_vzx, &r.m_sxx_x, &r.m_szz_z,
                       &r.m_sxz_x, &r.m_sxz_z, &r.m2_vxx, &r.m2_vzz, &r.m2_vxz, &r.m2_vzx};
@@ -1597,9 +1597,19 @@ int32_t sfd_run(sfd_handle* h, int64_t nsteps) {
       for (int q = 0; q < 17; ++q) std::swap(*at[q], r.out[q]);
       h->cur ^= 1;
     }
-    for (int m = 0; m < 4 && (n & 1); ++m)  // the in-place variables have one copy that stays
-      CK(cudaMemcpyAsync(h->mc(4 + m, 0), h->base + L.off_memS[m], sizeof(float) * L.mem_sz[4 + m],
-                         cudaMemcpyDeviceToDevice, h->stream));
+    // arrays first .. last lie back to back, in every copy
+    auto copy = [&](float* dst, const float* src, int first, int last) {
+      return cudaMemcpyAsync(dst, src, L.off_mem[last] - L.off_mem[first] + sizeof(float) * L.mem_sz[last],
+                             cudaMemcpyDeviceToDevice, h->stream);
+    };
+    if (n & 1) CK(copy(h->mc(4, 0), (const float*)(h->base + L.off_memS[0]), 4, 7));  // their one copy that stays
+    if ((n ^ nsteps) & 1) {  // into the copy that one launch a step would leave the state in
+      const int p = h->cur, q = 1 - p;
+      CK(cudaMemcpyAsync(h->fc(0, q), h->fc(0, p), sizeof(float) * L.fsz * 5, cudaMemcpyDeviceToDevice, h->stream));
+      CK(copy(h->mc(0, q), h->mc(0, p), 0, 3));
+      CK(copy(h->mc(8, q), h->mc(8, p), 8, 11));
+      h->cur = q;
+    }
     reduce_norms(h);
     CK(cudaGetLastError());
     h->step += nsteps;

@@ -35,7 +35,7 @@ extern __shared__ __align__(16) float em2_smem[];
 struct Em2Tile {
   int ox0, ox1, oz0, oz1;      // owned cells
   int bx, bz, xend, kend;      // frame
-  int wlo, wh0;                // warps below wlo and from wh0 on hold a z-strip row
+  int wlo, wh0;                // warps below wlo and from wh0 on hold a row that rounds dEz/dx (em2_rounded_z)
   int xlo, xh0, nxl;           // lanes below xlo and from xh0 on hold an x-strip cell; their number
   int zn;                      // frame rows in a z strip
   int hS;                      // floats of a field of the halo
@@ -53,7 +53,7 @@ struct Em2Tile {
 // step's state dumped, the handle's state kept); 2: a run that also saves
 // checkpoints; kStream: at most kTileHalo steps from one copy of the state to
 // the other, with no hand-over.  EDGE: the frame holds CPML strip or boundary
-// cells.  XS: it holds x-strip cells.
+// cells.  XS: it holds x-strip cells or columns that round dEz/dx (em2_rounded_x).
 //
 // Nothing updates Hy in row NZ - 1 and column NX - 1 or the memory variables
 // there (:249-295), and no update reads them: the registers' values are left
@@ -140,7 +140,7 @@ __device__ __forceinline__ void em2_run_tile(const Em2Resident& a, Em2Tile& G, i
     G.bx = bx; G.bz = bz; G.xend = xend; G.kend = kend;
     G.zn = max(min(W, kend) - bz, 0) + max(kend - max(NZ - W, bz), 0);
     G.wlo = (max(min(W, kend) - bz, 0) + RB - 1) / RB;
-    G.wh0 = max((max(NZ - W, bz) - bz) / RB, G.wlo);
+    G.wh0 = max((max(NZ - max(W, 2), bz) - bz) / RB, G.wlo);
     G.xlo = max((min(W, xend) - bx + 3) / 4, 0);
     G.xh0 = max((NX - W - bx) / 4, G.xlo);
     G.nxl = G.xlo + max((xend - bx + 3) / 4 - G.xh0, 0);
@@ -182,6 +182,14 @@ __device__ __forceinline__ void em2_run_tile(const Em2Resident& a, Em2Tile& G, i
     }
   }
   __syncthreads();
+  // this warp's rows, and whether this lane's columns, round dEz/dx (em2_rounded)
+  unsigned rounded = 0;
+  const bool roundx = XS && em2_rounded_x(bx + 4 * lane, NX, W);
+  if (EDGE)
+#pragma unroll
+    for (int j = 0; j < RB; ++j)
+      if (em2_rounded_z(bz + warp * RB + j, NZ, W)) rounded |= 1u << j;
+  const unsigned roundall = roundx ? ~0u : rounded;
   constexpr bool xs = XS;                                                                  // the tile has x-strip lanes ...
   const bool xsl = xs && nr > 0 && bx + 4 * lane < xend && (lane < G.xlo || lane >= G.xh0);  // ... and this is one
   const bool zw = EDGE && nr > 0 && (warp < G.wlo || warp >= G.wh0);                       // this warp has a z-strip row
@@ -446,7 +454,7 @@ __device__ __forceinline__ void em2_run_tile(const Em2Resident& a, Em2Tile& G, i
           float4 p = lds4(em2_smem + oZ + 2 * j * kCols);
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            el(p, e) = __fmaf_rn(rt.y, el(p, e), __fmul_rn(rt.z, el(dEx, e)));
+            el(p, e) = __fmaf_rn(rt.z, el(dEx, e), __fmul_rn(rt.y, el(p, e)));
             el(v, e) = __fadd_rn(el(v, e), el(p, e));
           }
           sts4(em2_smem + oZ + 2 * j * kCols, p);
@@ -454,17 +462,25 @@ __device__ __forceinline__ void em2_run_tile(const Em2Resident& a, Em2Tile& G, i
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           el(dEz, e) = __fsub_rn(e < 3 ? el(ez[j], e + 1) : ezn, el(ez[j], e));
-          el(v, e) = __fmaf_rn(el(dEz, e), el(ik, e), el(v, e));
         }
+        float4 p = zero4;
         if (xs) {
-          float4 p = zero4;
           if (xsl) p = lds4(em2_smem + oX + 2 * j * sX);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            el(p, e) = __fmaf_rn(el(xb, e), el(p, e), __fmul_rn(el(xa, e), el(dEz, e)));
-            el(v, e) = __fadd_rn(el(v, e), el(p, e));
-          }
+          for (int e = 0; e < 4; ++e) el(p, e) = __fmaf_rn(el(xb, e), el(p, e), __fmul_rn(el(xa, e), el(dEz, e)));
           if (xsl) sts4(em2_smem + oX + 2 * j * sX, p);
+        }
+        // dEz/dx, rounded or fused into the sum (em2_rounded; where it is fused, p is
+        // zero).  A select: two forms of the loop, or a branch a row, cost 4 to 7 %
+        // of a step of 1040 x 540 cells, this 1 %; the mask alone costs frames of two
+        // and four rows a warp 1 to 4 % more, the other way those of one and three.
+        const bool round = RB & 1 ? roundall >> j & 1u : roundx || (rounded >> j & 1u);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float fused = __fmaf_rn(el(dEz, e), el(ik, e), el(v, e));
+          float t = __fmul_rn(el(dEz, e), el(ik, e));
+          if (xs) t = __fadd_rn(t, el(p, e));
+          el(v, e) = (ZS || xs) && round ? __fadd_rn(t, el(v, e)) : fused;
         }
 #pragma unroll
         for (int e = 0; e < 4; ++e) el(hy[j], e) = __fmaf_rn(a.dbH, el(v, e), el(hy[j], e));
@@ -500,7 +516,7 @@ __device__ __forceinline__ void em2_run_tile(const Em2Resident& a, Em2Tile& G, i
             float4 p = lds4(em2_smem + oZ + (2 * j + 1) * kCols);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-              el(p, e) = __fmaf_rn(rt.y, el(p, e), __fmul_rn(rt.z, el(dH, e)));
+              el(p, e) = __fmaf_rn(rt.z, el(dH, e), __fmul_rn(rt.y, el(p, e)));
               el(d, e) = __fadd_rn(el(d, e), el(p, e));
             }
             sts4(em2_smem + oZ + (2 * j + 1) * kCols, p);

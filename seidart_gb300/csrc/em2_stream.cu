@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(32 * kWarps, 16 / kWarps)
   const int4 te = make_int4(cut_x(NX, c, ntx), cut_x(NX, c + 1, ntx), cut_z(NZ, r, nbz), cut_z(NZ, r + 1, nbz));
   const int bx = max(te.x - kTileHalo, 0), xend = min(NX, te.y + kTileHalo);
   const int bz = max(te.z - kTileHalo, 0), kend = min(NZ, te.w + kTileHalo);
-  const bool xs = bx < W || xend > NX - W;
+  const bool xs = bx < max(W, 1) || xend > NX - max(W, 2);
   const bool edge = xs || bx < 1 || xend > NX - 2 || bz < max(W, 1) || kend > NZ - max(W, 2);
   if (!edge) em2_run_tile<RB, kStream, false, false>(a, G, te);
   else if (!xs) em2_run_tile<RB, kStream, true, false>(a, G, te);
@@ -73,7 +73,7 @@ cudaError_t em2_stream_prepare(int NX, int NZ, int W, StreamPlan* out) {
   for (int r = 0; r < out->nbz; ++r) {
     const int bz = std::max(cut_z(NZ, r, out->nbz) - kTileHalo, 0), kend = std::min(NZ, cut_z(NZ, r + 1, out->nbz) + kTileHalo);
     const int wlo = (std::max(std::min(W, kend) - bz, 0) + kRows - 1) / kRows;
-    const int wh0 = std::max((std::max(NZ - W, bz) - bz) / kRows, wlo);
+    const int wh0 = std::max((std::max(NZ - std::max(W, 2), bz) - bz) / kRows, wlo);
     zrows = std::max(zrows, kRows * (wlo + std::max((kend - bz + kRows - 1) / kRows - wh0, 0)));
   }
   for (int c = 0; c < out->ntx; ++c) {

@@ -29,6 +29,15 @@ __device__ __forceinline__ float4 fld4(const float* p) {
 // ---------------------------------------------------------------------------
 // electromag2
 
+// Every product and sum of the update names its rounding, as in the tiles of
+// several steps (em2_run.cuh): a cell gets the same bits from either.
+
+// A memory variable's next value, of an x and of a z strip.
+__device__ __forceinline__ float em2_psi_x(float b, float p, float ad, float d) { return __fmaf_rn(b, p, __fmul_rn(ad, d)); }
+__device__ __forceinline__ float em2_psi_z(float b, float p, float ad, float d) { return __fmaf_rn(ad, d, __fmul_rn(b, p)); }
+// A field's: ca f + cb d.
+__device__ __forceinline__ float em2_next(float ca, float f, float cb, float d) { return __fmaf_rn(ca, f, __fmul_rn(cb, d)); }
+
 // Hy at (i, k) after the H half-step, from the old state
 // (electromagfdtd.f95:249-262).  Valid for i <= NX-2, k <= NZ-2.
 template <bool RO>
@@ -37,20 +46,21 @@ __device__ __forceinline__ float em2_h_cell(const Em2Step& a, int i, int k, floa
   const int P = a.P, W = a.W;
   const int c = k * P + i;
   const float dEx = fld<RO>(a.Ex0 + c + P) - fld<RO>(a.Ex0 + c);
-  float vz = dEx * __ldg(a.Z.ik + k);
+  float vz = __fmul_rn(dEx, __ldg(a.Z.ik + k));
   zs = in_strip(k, a.NZ, W);
   if (zs) {
-    pz = __ldg(a.Z.b + k) * fld<RO>(a.mExz0 + strip_idx(k, a.NZ, W) * P + i) + __ldg(a.Z.ad + k) * dEx;
-    vz += pz;
+    pz = em2_psi_z(__ldg(a.Z.b + k), fld<RO>(a.mExz0 + strip_idx(k, a.NZ, W) * P + i), __ldg(a.Z.ad + k), dEx);
+    vz = __fadd_rn(vz, pz);
   }
-  const float dEz = fld<RO>(a.Ez0 + c + 1) - fld<RO>(a.Ez0 + c);
-  float vx = dEz * __ldg(a.X.ik + i);
+  const float dEz = fld<RO>(a.Ez0 + c + 1) - fld<RO>(a.Ez0 + c), ik = __ldg(a.X.ik + i);
+  float vx = __fmul_rn(dEz, ik);
   xs = in_strip(i, a.NX, W);
   if (xs) {
-    px = __ldg(a.X.b + i) * fld<RO>(a.mEzx0 + k * (2 * W) + strip_idx(i, a.NX, W)) + __ldg(a.X.ad + i) * dEz;
-    vx += px;
+    px = em2_psi_x(__ldg(a.X.b + i), fld<RO>(a.mEzx0 + k * (2 * W) + strip_idx(i, a.NX, W)), __ldg(a.X.ad + i), dEz);
+    vx = __fadd_rn(vx, px);
   }
-  return fld<RO>(a.Hy0 + c) + a.dbH * (vx + vz);
+  const float v = em2_rounded(i, k, a.NX, a.NZ, W) ? __fadd_rn(vx, vz) : __fmaf_rn(dEz, ik, vz);
+  return __fmaf_rn(a.dbH, v, fld<RO>(a.Hy0 + c));
 }
 
 __device__ __forceinline__ float4 ld4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
@@ -100,26 +110,27 @@ __device__ __forceinline__ void em2_tile(const Em2Step& a, int t, int bx, int by
     const int zrow = (zs ? strip_idx(k, NZ, W) : 0) * P + i0;
     const float4 pz0 = (zs && active) ? fld4<RO>(a.mExz0 + zrow) : zero4;
     const float ikz = __ldg(a.Z.ik + k), adz = __ldg(a.Z.ad + k), bz = __ldg(a.Z.b + k);
+    const bool rounded = em2_rounded(i0, k, NX, NZ, W);
     float4 pz1 = pz0, hy1 = hy;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const int i = i0 + e;
       if (i <= NX - 2) {
         const float dEx = el(exn, e) - el(ex, e);
-        float vz = dEx * ikz;
+        float vz = __fmul_rn(dEx, ikz);
         if (zs) {
-          el(pz1, e) = bz * el(pz0, e) + adz * dEx;
-          vz += el(pz1, e);
+          el(pz1, e) = em2_psi_z(bz, el(pz0, e), adz, dEx);
+          vz = __fadd_rn(vz, el(pz1, e));
         }
         const float dEz = (e < 3 ? el(ez, e + 1) : ez_next) - el(ez, e);
-        float vx = dEz * el(ikx4, e);
+        float vx = __fmul_rn(dEz, el(ikx4, e));
         if (in_strip(i, NX, W)) {
           const int m = k * (2 * W) + strip_idx(i, NX, W);
-          const float px = el(bx4, e) * fld<RO>(a.mEzx0 + m) + el(adx4, e) * dEz;
+          const float px = em2_psi_x(el(bx4, e), fld<RO>(a.mEzx0 + m), el(adx4, e), dEz);
           if (own) a.mEzx1[m] = px;
-          vx += px;
+          vx = __fadd_rn(vx, px);
         }
-        el(hv, e) = el(hy, e) + a.dbH * (vx + vz);
+        el(hv, e) = __fmaf_rn(a.dbH, rounded ? __fadd_rn(vx, vz) : __fmaf_rn(dEz, el(ikx4, e), vz), el(hy, e));
         const bool edge = (i == 0) | (i == NX - 2) | (k == 0) | (k == NZ - 2);  // :314-317
         el(hy1, e) = edge ? 0.0f : el(hv, e);
       } else {
@@ -159,10 +170,8 @@ __device__ __forceinline__ void em2_tile(const Em2Step& a, int t, int bx, int by
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const float dEx = el(exn, e) - el(ex, e);
-        const float vz = dEx * ikz;
         const float dEz = (e < 3 ? el(ez, e + 1) : ez_next) - el(ez, e);
-        const float vx = dEz * el(ikx4, e);
-        el(hv[r], e) = el(hy, e) + a.dbH * (vx + vz);
+        el(hv[r], e) = __fmaf_rn(a.dbH, __fmaf_rn(dEz, el(ikx4, e), __fmul_rn(dEx, ikz)), el(hy, e));
       }
     }
 #pragma unroll
@@ -235,9 +244,9 @@ __device__ __forceinline__ void em2_tile(const Em2Step& a, int t, int bx, int by
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const float dHz = el(h, e) - el(hm, e);
-        const float exv = el(cax, e) * el(ex, e) + el(cbx, e) * (dHz * ikzh);
+        const float exv = em2_next(el(cax, e), el(ex, e), el(cbx, e), __fmul_rn(dHz, ikzh));
         const float dHx = el(h, e) - (e == 0 ? hl : el(h, e > 0 ? e - 1 : 0));
-        const float ezv = el(caz, e) * el(ez, e) + el(cbz, e) * (dHx * el(ikxh4, e));
+        const float ezv = em2_next(el(caz, e), el(ez, e), el(cbz, e), __fmul_rn(dHx, el(ikxh4, e)));
         el(ex, e) = exv;
         el(ez, e) = ezv;
         norm = fmaxf(norm, norm_monitor(exv, ezv));
@@ -275,23 +284,23 @@ __device__ __forceinline__ void em2_tile(const Em2Step& a, int t, int bx, int by
         float exv = el(ex, e), ezv = el(ez, e);
         if (i <= NX - 2 && k >= 1 && k <= NZ - 2) {  // :273-283
           const float dH = el(h, e) - el(hm, e);
-          float d = dH * ikzh;
+          float d = __fmul_rn(dH, ikzh);
           if (zs) {
-            el(pc1, e) = bzh * el(pc0, e) + adzh * dH;
-            d += el(pc1, e);
+            el(pc1, e) = em2_psi_z(bzh, el(pc0, e), adzh, dH);
+            d = __fadd_rn(d, el(pc1, e));
           }
-          exv = el(cax, e) * exv + el(cbx, e) * d;
+          exv = em2_next(el(cax, e), exv, el(cbx, e), d);
         }
         if (k <= NZ - 2 && i >= 1 && i <= NX - 2) {  // :285-295
           const float dH = el(h, e) - (e == 0 ? hl : el(h, e - 1));
-          float d = dH * el(ikxh4, e);
+          float d = __fmul_rn(dH, el(ikxh4, e));
           if (in_strip(i, NX, W)) {
             const int m = k * (2 * W) + strip_idx(i, NX, W);
-            const float psi = el(bxh4, e) * a.mHyx0[m] + el(adxh4, e) * dH;
+            const float psi = em2_psi_x(el(bxh4, e), a.mHyx0[m], el(adxh4, e), dH);
             a.mHyx[m] = psi;
-            d += psi;
+            d = __fadd_rn(d, psi);
           }
-          ezv = el(caz, e) * ezv + el(cbz, e) * d;
+          ezv = em2_next(el(caz, e), ezv, el(cbz, e), d);
         }
         if (i == a.io.si && k == a.io.sk) {  // :300-301
           exv += a.io.src[t];

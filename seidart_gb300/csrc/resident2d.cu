@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(32 * kEm2MaxWarps, 1) em2_resident_kernel(cons
   const int4 t = a.plan.tile[blockIdx.x];
   const int4 te = make_int4(t.x & 0xffff, t.x >> 16, t.y & 0xffff, t.y >> 16);
   if (t.z == 0) em2_run_tile<RB, MODE, false, false>(a, G, te);
-  else if (t.z == 1) em2_run_tile<RB, MODE, true, false>(a, G, te);
+  else if (t.z == 1 && te.y + kTileHalo <= a.NX - 2) em2_run_tile<RB, MODE, true, false>(a, G, te);
   else em2_run_tile<RB, MODE, true, true>(a, G, te);
 }
 

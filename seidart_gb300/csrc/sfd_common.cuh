@@ -93,6 +93,20 @@ __device__ __forceinline__ float norm_monitor(float a, float b, float c) {
   return (m <= 1e24f) ? m : nan_to_inf(norm3df(a, b, c));
 }
 
+// Whether electromag2 rounds dEz/dx before it adds it to dEx/dz in Hy's update
+// at cell (i, k); elsewhere the product is fused into the sum.  Rounded: where a
+// row, or a group of four columns, has cells of a strip or of a Dirichlet plane.
+// A property of the cell alone, so that every kernel gives a cell the same bits.
+__host__ __device__ __forceinline__ bool em2_rounded_x(int i, int NX, int W) {
+  return (i & ~3) < max(W, 1) || (i | 3) >= NX - max(W, 2);
+}
+__host__ __device__ __forceinline__ bool em2_rounded_z(int k, int NZ, int W) {
+  return k < max(W, 1) || k >= NZ - max(W, 2);
+}
+__host__ __device__ __forceinline__ bool em2_rounded(int i, int k, int NX, int NZ, int W) {
+  return em2_rounded_x(i, NX, W) || em2_rounded_z(k, NZ, W);
+}
+
 // Block-wide max of v (every thread of the block must call it); thread 0 then
 // folds it into this block's slot.  No atomics: each block owns its slot.
 __device__ __forceinline__ void block_norm_to_slot(float v, float* slots, int slot) {

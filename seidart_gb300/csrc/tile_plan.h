@@ -11,7 +11,7 @@ namespace sfd {
 // The frame of a tile of `cells` cells a lane with `halo` cells of halo.
 struct Frame {
   int rows, own, zlo, zhi, xlanes;  // rows, owned ones, those of the low and the high z strip, lanes with x-strip cells
-  int zhi0;                         // first row of the high z strip
+  int zhi0;                         // first row of the high z strip, of two rows at least
   bool edge;                        // it holds strip or boundary cells
 };
 
@@ -22,7 +22,7 @@ inline Frame frame_of(int NX, int NZ, int W, int cells, int halo, int ox0, int o
   f.rows = kend - bz;
   f.own = oz1 - oz0;
   f.zlo = std::max(std::min(W, kend) - bz, 0);
-  f.zhi0 = std::max(NZ - W, bz) - bz;
+  f.zhi0 = std::max(NZ - std::max(W, 2), bz) - bz;
   f.zhi = std::max(kend - std::max(NZ - W, bz), 0);
   const int xlo = std::max((std::min(W, xend) - bx + cells - 1) / cells, 0);
   const int xh0 = std::max((NX - W - bx) / cells, xlo);

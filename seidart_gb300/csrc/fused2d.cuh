@@ -324,6 +324,16 @@ __device__ __forceinline__ void em2_tile(const Em2Step& a, int t, int bx, int by
 // ---------------------------------------------------------------------------
 // seismic2
 
+// Every product and sum names its rounding, as in the tiles of several steps
+// (s2_run.cuh): a cell gets the same bits from either.
+
+// A memory variable's next value.
+__device__ __forceinline__ float s2_psi(float b, float m, float ad, float d) { return __fmaf_rn(b, m, __fmul_rn(ad, d)); }
+// A stress's: its rate a dx + b dz + c shear added.
+__device__ __forceinline__ float s2_stress(float s, float a, float dx, float b, float dz, float c, float shear) {
+  return __fadd_rn(s, __fmaf_rn(c, shear, __fmaf_rn(a, dx, __fmul_rn(b, dz))));
+}
+
 struct S2Stress {
   float sxx, szz, sxz;
   float mvxx, mvzx, mvzz, mvxz;  // velocity-gradient memory of the first stress loop (legacy: of both)
@@ -376,22 +386,22 @@ __device__ __forceinline__ S2Stress seis2_stress_cell(const Seis2Step& a, int i,
     const float d_vx_z = vx0 - fld<RO>(a.vx0 + c - P);
     if (o.xs) {
       const float bq = a.legacy ? __ldg(a.q3 + k) : __ldg(a.X.bh + i);  // b_x_half(j) as :255, or (i)
-      o.mvxx = bq * o.mvxx + __ldg(a.X.adh + i) * d_vx_x;
-      o.mvzx = __ldg(a.X.b + i) * o.mvzx + __ldg(a.X.ad + i) * d_vz_x;
+      o.mvxx = s2_psi(bq, o.mvxx, __ldg(a.X.adh + i), d_vx_x);
+      o.mvzx = s2_psi(__ldg(a.X.b + i), o.mvzx, __ldg(a.X.ad + i), d_vz_x);
     }
     if (o.zs) {
-      o.mvzz = __ldg(a.Z.b + k) * o.mvzz + __ldg(a.Z.ad + k) * d_vz_z;
-      o.mvxz = __ldg(a.Z.bh + k) * o.mvxz + __ldg(a.Z.adh + k) * d_vx_z;
+      o.mvzz = s2_psi(__ldg(a.Z.b + k), o.mvzz, __ldg(a.Z.ad + k), d_vz_z);
+      o.mvxz = s2_psi(__ldg(a.Z.bh + k), o.mvxz, __ldg(a.Z.adh + k), d_vx_z);
     }
-    const float dvx_dx = d_vx_x * ikxh + o.mvxx;
-    const float dvz_dz = d_vz_z * ikz + o.mvzz;
-    const float dvz_dx = d_vz_x * ikx + o.mvzx;
-    const float dvx_dz = d_vx_z * ikzh + o.mvxz;
+    const float dvx_dx = __fmaf_rn(d_vx_x, ikxh, o.mvxx);
+    const float dvz_dz = __fmaf_rn(d_vz_z, ikz, o.mvzz);
+    const float dvz_dx = __fmaf_rn(d_vz_x, ikx, o.mvzx);
+    const float dvx_dz = __fmaf_rn(d_vx_z, ikzh, o.mvxz);
     const float A11 = __ldg(a.A11 + c), A13 = __ldg(a.A13 + c), A15 = __ldg(a.A15 + c);
     const float A33 = __ldg(a.A33 + c), A35 = __ldg(a.A35 + c);
-    const float shear = dvz_dx + dvx_dz;
-    o.sxx = o.sxx + (A11 * dvx_dx + A13 * dvz_dz + A15 * shear);
-    o.szz = o.szz + (A13 * dvx_dx + A33 * dvz_dz + A35 * shear);
+    const float shear = __fadd_rn(dvz_dx, dvx_dz);
+    o.sxx = s2_stress(o.sxx, A11, dvx_dx, A13, dvz_dz, A15, shear);
+    o.szz = s2_stress(o.szz, A13, dvx_dx, A33, dvz_dz, A35, shear);
   }
   if (loop2) {
     const float d_vx_x = vx0 - fld<RO>(a.vx0 + c - 1);
@@ -401,19 +411,19 @@ __device__ __forceinline__ S2Stress seis2_stress_cell(const Seis2Step& a, int i,
     float mxx = own2 ? o.nvxx : o.mvxx, mzx = own2 ? o.nvzx : o.mvzx;
     float mzz = own2 ? o.nvzz : o.mvzz, mxz = own2 ? o.nvxz : o.mvxz;
     if (o.xs) {
-      mxx = __ldg(a.X.bh + i) * mxx + __ldg(a.X.adh + i) * d_vx_x;
-      mzx = __ldg(a.X.b + i) * mzx + __ldg(a.X.ad + i) * d_vz_x;
+      mxx = s2_psi(__ldg(a.X.bh + i), mxx, __ldg(a.X.adh + i), d_vx_x);
+      mzx = s2_psi(__ldg(a.X.b + i), mzx, __ldg(a.X.ad + i), d_vz_x);
     }
     if (o.zs) {
-      mzz = __ldg(a.Z.b + k) * mzz + __ldg(a.Z.ad + k) * d_vz_z;
-      mxz = __ldg(a.Z.bh + k) * mxz + __ldg(a.Z.adh + k) * d_vx_z;
+      mzz = s2_psi(__ldg(a.Z.b + k), mzz, __ldg(a.Z.ad + k), d_vz_z);
+      mxz = s2_psi(__ldg(a.Z.bh + k), mxz, __ldg(a.Z.adh + k), d_vx_z);
     }
-    const float dvx_dx = d_vx_x * ikxh + mxx;
-    const float dvz_dz = d_vz_z * ikz + mzz;
-    const float dvz_dx = d_vz_x * ikx + mzx;
-    const float dvx_dz = d_vx_z * ikzh + mxz;
-    o.sxz = o.sxz + (__ldg(a.B15 + c) * dvx_dx + __ldg(a.B35 + c) * dvz_dz +
-                     __ldg(a.B55 + c) * (dvz_dx + dvx_dz));
+    const float dvx_dx = __fmaf_rn(d_vx_x, ikxh, mxx);
+    const float dvz_dz = __fmaf_rn(d_vz_z, ikz, mzz);
+    const float dvz_dx = __fmaf_rn(d_vz_x, ikx, mzx);
+    const float dvx_dz = __fmaf_rn(d_vx_z, ikzh, mxz);
+    o.sxz = s2_stress(o.sxz, __ldg(a.B15 + c), dvx_dx, __ldg(a.B35 + c), dvz_dz, __ldg(a.B55 + c),
+                      __fadd_rn(dvz_dx, dvx_dz));
     if (own2) { o.nvxx = mxx; o.nvzx = mzx; o.nvzz = mzz; o.nvxz = mxz; }
     else { o.mvxx = mxx; o.mvzx = mzx; o.mvzz = mzz; o.mvxz = mxz; }
   }
@@ -445,18 +455,18 @@ __device__ __forceinline__ void seis2_stress_plain(const Seis2Step& a, int i, in
   szz = fld<RO>(a.szz0 + c);
   sxz = fld<RO>(a.sxz0 + c);
   {  // :247-283
-    const float dvx_dx = (vxr - vx0) * ikxh, dvz_dz = (vz0 - vzu) * ikz;
-    const float dvz_dx = (vzr - vz0) * ikx, dvx_dz = (vx0 - vxu) * ikzh;
+    const float dvx_dx = __fmul_rn(vxr - vx0, ikxh), dvz_dz = __fmul_rn(vz0 - vzu, ikz);
+    const float dvz_dx = __fmul_rn(vzr - vz0, ikx), dvx_dz = __fmul_rn(vx0 - vxu, ikzh);
     const float A11 = __ldg(a.A11 + c), A13 = __ldg(a.A13 + c), A15 = __ldg(a.A15 + c);
     const float A33 = __ldg(a.A33 + c), A35 = __ldg(a.A35 + c);
-    const float shear = dvz_dx + dvx_dz;
-    sxx = sxx + (A11 * dvx_dx + A13 * dvz_dz + A15 * shear);
-    szz = szz + (A13 * dvx_dx + A33 * dvz_dz + A35 * shear);
+    const float shear = __fadd_rn(dvz_dx, dvx_dz);
+    sxx = s2_stress(sxx, A11, dvx_dx, A13, dvz_dz, A15, shear);
+    szz = s2_stress(szz, A13, dvx_dx, A33, dvz_dz, A35, shear);
   }
   {  // :285-312
-    const float dvx_dx = (vx0 - vxl) * ikxh, dvz_dz = (vzd - vz0) * ikz;
-    const float dvz_dx = (vz0 - vzl) * ikx, dvx_dz = (vxd - vx0) * ikzh;
-    sxz = sxz + (__ldg(a.B15 + c) * dvx_dx + __ldg(a.B35 + c) * dvz_dz + __ldg(a.B55 + c) * (dvz_dx + dvx_dz));
+    const float dvx_dx = __fmul_rn(vx0 - vxl, ikxh), dvz_dz = __fmul_rn(vzd - vz0, ikz);
+    const float dvz_dx = __fmul_rn(vz0 - vzl, ikx), dvx_dz = __fmul_rn(vxd - vx0, ikzh);
+    sxz = s2_stress(sxz, __ldg(a.B15 + c), dvx_dx, __ldg(a.B35 + c), dvz_dz, __ldg(a.B55 + c), __fadd_rn(dvz_dx, dvx_dz));
   }
 }
 
@@ -562,15 +572,17 @@ __device__ __forceinline__ void seis2_tile(const Seis2Step& a, int t, int bx, in
       const int k = z0 + ty + 8 * r;
       const int c = k * P + i;
       const int kk = ty + 8 * r + 1, ii = tx + 1;
-      const float v1 = (sS[0][kk][ii] - sS[0][kk][ii - 1]) * ikx, v2 = (sS[2][kk][ii] - sS[2][kk - 1][ii]) * __ldg(a.Z.ik + k);
-      const float w1 = (sS[2][kk][ii + 1] - sS[2][kk][ii]) * ikxh, w2 = (sS[1][kk + 1][ii] - sS[1][kk][ii]) * __ldg(a.Z.ikh + k);
+      const float v1 = __fmul_rn(sS[0][kk][ii] - sS[0][kk][ii - 1], ikx);
+      const float v2 = __fmul_rn(sS[2][kk][ii] - sS[2][kk - 1][ii], __ldg(a.Z.ik + k));
+      const float w1 = __fmul_rn(sS[2][kk][ii + 1] - sS[2][kk][ii], ikxh);
+      const float w2 = __fmul_rn(sS[1][kk + 1][ii] - sS[1][kk][ii], __ldg(a.Z.ikh + k));
       float vx = fld<RO>(a.vx0 + c), vz = fld<RO>(a.vz0 + c);
       if (a.atten) {
-        vx *= __ldg(a.gxp + c);
-        vz *= __ldg(a.gzp + c);
+        vx = __fmul_rn(vx, __ldg(a.gxp + c));
+        vz = __fmul_rn(vz, __ldg(a.gzp + c));
       }
-      vx = vx + (v1 + v2) * __ldg(a.dtrx + c);
-      vz = vz + (w1 + w2) * __ldg(a.dtrz + c);
+      vx = __fmaf_rn(__fadd_rn(v1, v2), __ldg(a.dtrx + c), vx);
+      vz = __fmaf_rn(__fadd_rn(w1, w2), __ldg(a.dtrz + c), vz);
       vxr[r] = vx;
       vzr[r] = vz;
       norm = fmaxf(norm, norm_monitor(vx, vz));
@@ -596,41 +608,41 @@ __device__ __forceinline__ void seis2_tile(const Seis2Step& a, int t, int bx, in
       if (k >= 1 && i >= 1) {  // vx loop, :317-336
         const float d1 = sS[0][kk][ii] - sS[0][kk][ii - 1];
         const float d2 = sS[2][kk][ii] - sS[2][kk - 1][ii];
-        float v1 = d1 * __ldg(a.X.ik + i), v2 = d2 * __ldg(a.Z.ik + k);
+        float v1 = __fmul_rn(d1, __ldg(a.X.ik + i)), v2 = __fmul_rn(d2, __ldg(a.Z.ik + k));
         if (xs) {
-          const float m = __ldg(a.X.b + i) * a.m_sxx_x[mx] + __ldg(a.X.ad + i) * d1;
+          const float m = s2_psi(__ldg(a.X.b + i), a.m_sxx_x[mx], __ldg(a.X.ad + i), d1);
           a.m_sxx_x[mx] = m;
-          v1 += m;
+          v1 = __fadd_rn(v1, m);
         }
         if (zs) {
-          const float m = __ldg(a.Z.b + k) * a.m_sxz_z[mz] + __ldg(a.Z.ad + k) * d2;
+          const float m = s2_psi(__ldg(a.Z.b + k), a.m_sxz_z[mz], __ldg(a.Z.ad + k), d2);
           a.m_sxz_z[mz] = m;
-          v2 += m;
+          v2 = __fadd_rn(v2, m);
         }
         if (interior) {
           vx = fld<RO>(a.vx0 + c);
-          if (a.atten) vx *= __ldg(a.gxp + c);
-          vx = vx + (v1 + v2) * __ldg(a.dtrx + c);
+          if (a.atten) vx = __fmul_rn(vx, __ldg(a.gxp + c));
+          vx = __fmaf_rn(__fadd_rn(v1, v2), __ldg(a.dtrx + c), vx);
         }
       }
       if (k <= NZ - 2 && i <= NX - 2) {  // vz loop, :338-357
         const float d1 = sS[2][kk][ii + 1] - sS[2][kk][ii];
         const float d2 = sS[1][kk + 1][ii] - sS[1][kk][ii];
-        float v1 = d1 * __ldg(a.X.ikh + i), v2 = d2 * __ldg(a.Z.ikh + k);
+        float v1 = __fmul_rn(d1, __ldg(a.X.ikh + i)), v2 = __fmul_rn(d2, __ldg(a.Z.ikh + k));
         if (xs) {
-          const float m = __ldg(a.X.bh + i) * a.m_sxz_x[mx] + __ldg(a.X.adh + i) * d1;
+          const float m = s2_psi(__ldg(a.X.bh + i), a.m_sxz_x[mx], __ldg(a.X.adh + i), d1);
           a.m_sxz_x[mx] = m;
-          v1 += m;
+          v1 = __fadd_rn(v1, m);
         }
         if (zs) {
-          const float m = __ldg(a.Z.bh + k) * a.m_szz_z[mz] + __ldg(a.Z.adh + k) * d2;
+          const float m = s2_psi(__ldg(a.Z.bh + k), a.m_szz_z[mz], __ldg(a.Z.adh + k), d2);
           a.m_szz_z[mz] = m;
-          v2 += m;
+          v2 = __fadd_rn(v2, m);
         }
         if (interior) {
           vz = fld<RO>(a.vz0 + c);
-          if (a.atten) vz *= __ldg(a.gzp + c);
-          vz = vz + (v1 + v2) * __ldg(a.dtrz + c);
+          if (a.atten) vz = __fmul_rn(vz, __ldg(a.gzp + c));
+          vz = __fmaf_rn(__fadd_rn(v1, v2), __ldg(a.dtrz + c), vz);
         }
       }
       if (i == a.io.si && k == a.io.sk) {  // :360-361

@@ -521,7 +521,9 @@ __device__ __forceinline__ void s2_run_tile(const Seis2Resident& a, S2Tile& G, i
       }
     }
   };
-  // The velocities of this warp's rows (:317-357)
+  // The velocities of this warp's rows (:317-357).  Both derivatives are rounded
+  // before they are added: next to a source they cancel, and a fused product
+  // leaves the other's rounding error in the velocity every step.
   auto velocity_rows = [&](auto zs_tag) {
     constexpr bool ZS = decltype(zs_tag)::value;
     const float2 sxzt = lds(kSS + (max(warp - 1, 0) * 2 + 1) * kSC + 2 * lane);
@@ -575,8 +577,8 @@ __device__ __forceinline__ void s2_run_tile(const Seis2Resident& a, S2Tile& G, i
         sts(oZ + (6 * j + 5) * kSC, m2);
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          el(d2, e) = __fmaf_rn(el(d2, e), rt.x, el(m2, e));
-          el(e2, e) = __fmaf_rn(el(e2, e), rt.y, el(n2, e));
+          el(d2, e) = __fadd_rn(__fmul_rn(el(d2, e), rt.x), el(m2, e));
+          el(e2, e) = __fadd_rn(__fmul_rn(el(e2, e), rt.y), el(n2, e));
         }
       } else {
 #pragma unroll
@@ -596,13 +598,13 @@ __device__ __forceinline__ void s2_run_tile(const Seis2Resident& a, S2Tile& G, i
       }
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        float s = __fmaf_rn(el(d1, e), el(ikx, e), el(d2, e)), t = __fmaf_rn(el(e1, e), el(ikxh, e), el(e2, e));
+        float s = __fmul_rn(el(d1, e), el(ikx, e)), t = __fmul_rn(el(e1, e), el(ikxh, e));
         if (XS) {
           s = __fadd_rn(s, el(m1, e));
           t = __fadd_rn(t, el(n1, e));
         }
-        el(vx[j], e) = __fmaf_rn(s, el(rx, e), el(vx[j], e));
-        el(vz[j], e) = __fmaf_rn(t, el(rz, e), el(vz[j], e));
+        el(vx[j], e) = __fmaf_rn(__fadd_rn(s, el(d2, e)), el(rx, e), el(vx[j], e));
+        el(vz[j], e) = __fmaf_rn(__fadd_rn(t, el(e2, e)), el(rz, e), el(vz[j], e));
       }
     }
   };

@@ -1,6 +1,7 @@
 // Streaming electromag2 runs: grids too large for the chip (and handles told to
 // stay off it) advance kTileHalo steps a launch, every launch reading one copy
-// of the state and writing the other.
+// of the state and writing the other; what is left of a run takes single steps
+// (fused2d.cu; sfd_api.cu says how many).
 //
 // The tiles are those of the on-chip run (em2_run.cuh): a CTA loads its frame --
 // the owned cells, four cells of halo, coefficients and strips' memory

@@ -2,8 +2,8 @@
 // scheme of electromag2 with complex permittivities, hence complex update
 // coefficients, fields and CPML memory variables.  Complex arrays are held
 // as separate real and imaginary planes (x fastest, pitch P), so each plane
-// streams like a real field.  Two kernels per step (SFD_FLAG_TWO_PASS; other
-// runs: em2c_stream.cu), as the two-pass electromag2 (em2.cu):
+// streams like a real field.  Two kernels per step (SFD_FLAG_TWO_PASS, and runs
+// of a step or two; the others: em2c_stream.cu), as the two-pass electromag2 (em2.cu):
 //   half1: Hy (:530-549) with the dEx/dz, dEz/dx memory variables; block
 //          (0,0) first records the receivers of the previous step;
 //   half2: Ex (:556-565), Ez (:567-576) with the dHy memory variables, the
@@ -40,6 +40,20 @@ __device__ __forceinline__ float norm_monitor_c(cf ex, cf ez) {
   return nan_to_inf(s * sqrtf(hypotf(w.r, w.i)));
 }
 
+// The streaming tiles' forms (em2c_stream.cu), bit for bit: s a + b; a memory
+// variable's next value; ca f + cb d.
+__device__ __forceinline__ cf cfma(float s, cf a, cf b) { return {__fmaf_rn(s, a.r, b.r), __fmaf_rn(s, a.i, b.i)}; }
+__device__ __forceinline__ cf tile_psi(float b, cf p, float ad, cf d) {
+  return cfma(b, p, {__fmul_rn(ad, d.r), __fmul_rn(ad, d.i)});
+}
+__device__ __forceinline__ cf tile_next(cf ca, cf f, cf cb, cf d) {
+  return {__fmaf_rn(ca.r, f.r, __fmaf_rn(-ca.i, f.i, __fmaf_rn(cb.r, d.r, -__fmul_rn(cb.i, d.i)))),
+          __fmaf_rn(ca.r, f.i, __fmaf_rn(ca.i, f.r, __fmaf_rn(cb.r, d.i, __fmul_rn(cb.i, d.r))))};
+}
+
+// T: rounded as the tiles round, for single steps between their launches; else the
+// two-pass form's own rounding.
+template <bool T>
 __global__ void __launch_bounds__(BX * BY) em2c_h_kernel(Em2cArgs a, int rel) {
   const Ctl* ctl = a.io.ctl;
   const int t = ctl->base + rel;
@@ -57,17 +71,19 @@ __global__ void __launch_bounds__(BX * BY) em2c_h_kernel(Em2cArgs a, int rel) {
   cf vz = cscale(a.Z.ik[k], dEx);
   if (in_strip(k, NZ, W)) {
     const size_t m = (size_t)strip_idx(k, NZ, W) * P + i;
-    const cf psi = cadd(cscale(a.Z.b[k], {a.mExz[0][m], a.mExz[1][m]}), cscale(a.Z.ad[k], dEx));
+    const cf p = {a.mExz[0][m], a.mExz[1][m]};
+    const cf psi = T ? tile_psi(a.Z.b[k], p, a.Z.ad[k], dEx) : cadd(cscale(a.Z.b[k], p), cscale(a.Z.ad[k], dEx));
     a.mExz[0][m] = psi.r;
     a.mExz[1][m] = psi.i;
     vz = cadd(vz, psi);
   }
   // dEz/dx, :538-540
   const cf dEz = {a.Ez[0][c + 1] - a.Ez[0][c], a.Ez[1][c + 1] - a.Ez[1][c]};
-  cf vx = cscale(a.X.ik[i], dEz);
+  cf vx = T ? cfma(a.X.ik[i], dEz, vz) : cscale(a.X.ik[i], dEz);
   if (in_strip(i, NX, W)) {
     const size_t m = (size_t)k * (2 * W) + strip_idx(i, NX, W);
-    const cf psi = cadd(cscale(a.X.b[i], {a.mEzx[0][m], a.mEzx[1][m]}), cscale(a.X.ad[i], dEz));
+    const cf p = {a.mEzx[0][m], a.mEzx[1][m]};
+    const cf psi = T ? tile_psi(a.X.b[i], p, a.X.ad[i], dEz) : cadd(cscale(a.X.b[i], p), cscale(a.X.ad[i], dEz));
     a.mEzx[0][m] = psi.r;
     a.mEzx[1][m] = psi.i;
     vx = cadd(vx, psi);
@@ -75,11 +91,12 @@ __global__ void __launch_bounds__(BX * BY) em2c_h_kernel(Em2cArgs a, int rel) {
   // the previous Hy on its Dirichlet edges is zero (they are zeroed after the E half, :595-598)
   const bool edge = (i == 0) | (i == NX - 2) | (k == 0) | (k == NZ - 2);
   const cf hy = edge ? cf{0.0f, 0.0f} : cf{a.Hy[0][c], a.Hy[1][c]};
-  const cf h = cadd(hy, cscale(a.dbH, cadd(vx, vz)));  // :543
+  const cf h = T ? cfma(a.dbH, vx, hy) : cadd(hy, cscale(a.dbH, cadd(vx, vz)));  // :543
   a.Hy[0][c] = h.r;
   a.Hy[1][c] = h.i;
 }
 
+template <bool T>
 __global__ void __launch_bounds__(BX * BY) em2c_e_kernel(Em2cArgs a, int rel) {
   const int t = a.io.ctl->base + rel;
   const int i = blockIdx.x * BX + threadIdx.x;
@@ -97,12 +114,14 @@ __global__ void __launch_bounds__(BX * BY) em2c_e_kernel(Em2cArgs a, int rel) {
         cf d = cscale(a.Z.ikh[k], dH);
         if (in_strip(k, NZ, W)) {
           const size_t m = (size_t)strip_idx(k, NZ, W) * P + i;
-          const cf psi = cadd(cscale(a.Z.bh[k], {a.mHyz[0][m], a.mHyz[1][m]}), cscale(a.Z.adh[k], dH));
+          const cf p = {a.mHyz[0][m], a.mHyz[1][m]};
+          const cf psi = T ? tile_psi(a.Z.bh[k], p, a.Z.adh[k], dH) : cadd(cscale(a.Z.bh[k], p), cscale(a.Z.adh[k], dH));
           a.mHyz[0][m] = psi.r;
           a.mHyz[1][m] = psi.i;
           d = cadd(d, psi);
         }
-        ex = cadd(cmul({a.CAx[0][c], a.CAx[1][c]}, ex), cmul({a.CBx[0][c], a.CBx[1][c]}, d));
+        const cf ca = {a.CAx[0][c], a.CAx[1][c]}, cb = {a.CBx[0][c], a.CBx[1][c]};
+        ex = T ? tile_next(ca, ex, cb, d) : cadd(cmul(ca, ex), cmul(cb, d));
       }
     }
     // Ez, :567-576 (k in [0, NZ-2], i in [1, NX-2])
@@ -113,12 +132,14 @@ __global__ void __launch_bounds__(BX * BY) em2c_e_kernel(Em2cArgs a, int rel) {
         cf d = cscale(a.X.ikh[i], dH);
         if (in_strip(i, NX, W)) {
           const size_t m = (size_t)k * (2 * W) + strip_idx(i, NX, W);
-          const cf psi = cadd(cscale(a.X.bh[i], {a.mHyx[0][m], a.mHyx[1][m]}), cscale(a.X.adh[i], dH));
+          const cf p = {a.mHyx[0][m], a.mHyx[1][m]};
+          const cf psi = T ? tile_psi(a.X.bh[i], p, a.X.adh[i], dH) : cadd(cscale(a.X.bh[i], p), cscale(a.X.adh[i], dH));
           a.mHyx[0][m] = psi.r;
           a.mHyx[1][m] = psi.i;
           d = cadd(d, psi);
         }
-        ez = cadd(cmul({a.CAz[0][c], a.CAz[1][c]}, ez), cmul({a.CBz[0][c], a.CBz[1][c]}, d));
+        const cf ca = {a.CAz[0][c], a.CAz[1][c]}, cb = {a.CBz[0][c], a.CBz[1][c]};
+        ez = T ? tile_next(ca, ez, cb, d) : cadd(cmul(ca, ez), cmul(cb, d));
       }
     }
     // Source, :581-582 (amplitudes already divided by the complex permittivity)
@@ -171,11 +192,13 @@ Launch em2c_launch(const Em2cArgs& a) {
 }
 
 void em2c_half1(const Em2cArgs& a, const Launch& L, int rel, cudaStream_t s) {
-  em2c_h_kernel<<<L.grid, L.block, 0, s>>>(a, rel);
+  if (a.as_tiles) em2c_h_kernel<true><<<L.grid, L.block, 0, s>>>(a, rel);
+  else em2c_h_kernel<false><<<L.grid, L.block, 0, s>>>(a, rel);
 }
 
 void em2c_half2(const Em2cArgs& a, const Launch& L, int rel, cudaStream_t s) {
-  em2c_e_kernel<<<L.grid, L.block, 0, s>>>(a, rel);
+  if (a.as_tiles) em2c_e_kernel<true><<<L.grid, L.block, 0, s>>>(a, rel);
+  else em2c_e_kernel<false><<<L.grid, L.block, 0, s>>>(a, rel);
 }
 
 void em2c_finalize(const Em2cArgs& a, int t_last, cudaStream_t s) { em2c_finalize_kernel<<<1, 256, 0, s>>>(a, t_last); }

@@ -247,8 +247,9 @@ struct StreamPlan {
 cudaError_t em2_stream_prepare(int NX, int NZ, int W, StreamPlan* out);
 void em2_stream_launch(const Em2Resident& a, const StreamPlan& plan, cudaStream_t s);
 
-// The same for seismic2 (s2_stream.cu), at most kS2Steps steps a launch.
-cudaError_t seis2_stream_prepare(int NX, int NZ, int W, StreamPlan* out);
+// The same for seismic2 (s2_stream.cu), at most kS2Steps steps a launch; and
+// whether a long run is faster so than in one launch a step.
+cudaError_t seis2_stream_prepare(int NX, int NZ, int W, StreamPlan* out, bool* faster);
 void seis2_stream_launch(const Seis2Resident& a, const StreamPlan& plan, cudaStream_t s);
 
 // Streaming electromag2c runs (em2c_stream.cu): at most kC2Halo steps a launch

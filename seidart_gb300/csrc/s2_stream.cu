@@ -1,6 +1,7 @@
 // Streaming seismic2 runs (corrected physics): grids too large for the chip (and
 // handles told to stay off it) advance kS2Steps steps a launch, every launch
-// reading one copy of the state and writing the other.
+// reading one copy of the state and writing the other, where that is faster than
+// single steps (fused2d.cu), which what is left of a run takes too.
 //
 // The tiles are those of the on-chip run (s2_run.cuh): a CTA loads its frame -- the
 // owned cells, kS2Halo cells of halo, coefficients and strips' memory variables
@@ -67,9 +68,18 @@ size_t tile_smem(int NX, int NZ, int W, int rb, int ntx, int nbz) {
 
 }  // namespace
 
-cudaError_t seis2_stream_prepare(int NX, int NZ, int W, StreamPlan* out) {
-  int dev = 0, optin = 0;
+// Tiles are worth it where they fill 0.7 of their waves (one CTA an SM): a launch of
+// one wave takes 23 us, of two 32, of three 43, whatever the last one holds, and a
+// single-pass step 7 us and 20 for a million cells.  (us a step so and so: 635 x 460
+// cells, 0.86 of one wave, 11.5 and 12.6; 723 x 549, 0.58 of two, 15.9 and 15.3;
+// 1036 x 501, 0.76 of two, 15.7 and 17.7; 897 x 907, 0.80 of three, 21.4 and 22.7.)
+// Grids of less than a wave run here only when told to stream.
+constexpr double kWorth = 0.7;
+
+cudaError_t seis2_stream_prepare(int NX, int NZ, int W, StreamPlan* out, bool* faster) {
+  int dev = 0, optin = 0, sms = 0;
   cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   if (e != cudaSuccess) return e;
   const size_t limit = (size_t)optin - sizeof(S2Tile) - 256;  // the static shared memory (and block_norm_to_slot's)
@@ -81,6 +91,9 @@ cudaError_t seis2_stream_prepare(int NX, int NZ, int W, StreamPlan* out) {
     out->smem = tile_smem(NX, NZ, W, out->rb, out->ntx, out->nbz);
     if (out->smem <= limit || out->rb == 2) break;
   }
+  const int waves = (out->ntx * out->nbz + sms - 1) / sms;
+  const double wave = (double)sms * (kSC - 2 * kS2Halo) * (kS2Warps * out->rb - 2 * kS2Halo);  // cells
+  *faster = waves == 1 || (double)NX * NZ > kWorth * waves * wave;
   return res_allow_max_smem((const void*)kernel_of(out->rb));
 }
 

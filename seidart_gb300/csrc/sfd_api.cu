@@ -380,6 +380,7 @@ bool bind_args(sfd_handle* h) {
       a.X = make_axis(h->axis(0), NX); a.Z = make_axis(h->axis(1), NZ);
       a.dbH = (float)(c.dt / kMu0);
       a.io = io;
+      a.as_tiles = streams_complex(c);
       h->launch = em2c_launch(a);
       break;
     }
@@ -676,14 +677,6 @@ int run_on_chip(sfd_handle* h, int64_t nsteps, unsigned long long limit_ns) {
   return SFD_OK;
 }
 
-// Launches of a streaming run that advances up to `most` steps a launch, from
-// copy to copy of the state: of the steps' parity, so that the state after the
-// run lies in the copy that one launch a step would leave it in.
-int64_t stream_launches(int64_t nsteps, int64_t most) {
-  const int64_t n = (nsteps + most - 1) / most;
-  return n + ((n ^ nsteps) & 1);
-}
-
 int ensure_graph(sfd_handle* h, int p) {
   if (h->graph[p]) return SFD_OK;
   cudaGraph_t g = nullptr;
@@ -709,6 +702,115 @@ void invalidate_graph(sfd_handle* h) {
   for (int p = 0; p < 2; ++p)
     if (h->graph[p]) { cudaGraphExecDestroy(h->graph[p]); h->graph[p] = nullptr; }
   if (h->adj_graph) { cudaGraphExecDestroy(h->adj_graph); h->adj_graph = nullptr; }
+}
+
+// nsteps steps in one launch each (two without the single-pass form), the last
+// of a run `done` steps into it.
+int run_steps(sfd_handle* h, int64_t nsteps, int done) {
+  const int64_t chunks = h->cap_stream && !done ? nsteps / kGraphSteps : 0;
+  const int rem = (int)(nsteps - chunks * kGraphSteps);
+  if (chunks > 0) {
+    int r = ensure_graph(h, h->single ? h->cur : 0);
+    if (r) return r;
+    for (int64_t q = 0; q < chunks; ++q) CK(cudaGraphLaunch(h->graph[h->single ? h->cur : 0], h->stream));
+  }
+  for (int s = done; s < done + rem; ++s) {
+    if (h->single) {
+      launch_step(h, h->cur, s, h->stream);
+      h->cur ^= 1;
+    } else {
+      launch_half(h, 0, s, h->stream);
+      launch_half(h, 1, s, h->stream);
+    }
+  }
+  if (nsteps > 0) launch_finalize(h, (int)(h->step + done + nsteps - 1), h->stream);
+  return SFD_OK;
+}
+
+// A streaming electromag2 run: launches of four steps in pairs, then of three, then
+// single steps.  Each launch goes from one copy of the state to the other, and so
+// many of them are of their steps' parity: the state ends in the copy that one
+// launch a step would leave it in.  (4040 x 3040 cells, us a run of 1, 2, 4, 5, 7
+// steps, set-up and norms included: 138, 245, 294, 399, 449; in the fewest launches
+// of that parity, single steps among them as launches of one, 165, 301, 325, 461,
+// 486.  300 x 200 cells: 19, 27, 33, 41, 43 and 22, 39, 41, 57, 60.)
+int em2_stream_run(sfd_handle* h, int64_t nsteps) {
+  StreamPlan plan;
+  int64_t done = 0;
+  if (nsteps >= 3) CK(em2_stream_prepare(h->cfg.nx, h->cfg.nz, h->cfg.npml, &plan));
+  while (nsteps - done >= 3) {
+    const int64_t left = nsteps - done;
+    const int steps = left >= 2 * kTileHalo || done % (2 * kTileHalo) == kTileHalo ? kTileHalo : 3;
+    const int q = 1 - h->cur;
+    Em2Resident r = resident_args(h, steps);
+    r.oEx = h->fc(0, q); r.oEz = h->fc(1, q); r.oHy = h->fc(2, q);
+    r.omExz = h->mc(0, q); r.omEzx = h->mc(1, q); r.omHyz = h->mc(2, q); r.omHyx = h->mc(3, q);
+    r.t0 += (int)done;
+    em2_stream_launch(r, plan, h->stream);
+    h->cur = q;
+    done += steps;
+  }
+  return run_steps(h, nsteps - done, (int)done);
+}
+
+// A streaming seismic2 run: launches of two steps in pairs, so that the state ends
+// in the copy that one launch a step would leave it in, then single steps.  (2040 x
+// 1540 cells, us a run of 1, 2, 3, 5 steps: 103, 188, 274, 397; in launches of two
+// and one with the state copied back 151, 199, 322, 434.)
+int seis2_stream_run(sfd_handle* h, int64_t nsteps) {
+  StreamPlan plan;
+  int64_t done = 0;
+  bool tiles = nsteps >= 2 * kS2Steps;
+  if (tiles) CK(seis2_stream_prepare(h->cfg.nx, h->cfg.nz, h->cfg.npml, &plan, &tiles));
+  tiles = tiles || (nsteps >= 2 * kS2Steps && nsteps < kGraphSteps);  // no graph of steps: 16 of 723 x 549 cells 284 us, 257 in tiles
+  if (tiles) {
+    Seis2Resident r = seis2_resident_args(h, kS2Steps);
+    float** at[17] = {&r.vx, &r.vz, &r.sxx, &r.szz, &r.sxz, &r.m_vxx, &r.m_vzz, &r.m_vxz, &r.m_vzx, &r.m_sxx_x, &r.m_szz_z,
+                      &r.m_sxz_x, &r.m_sxz_z, &r.m2_vxx, &r.m2_vzz, &r.m2_vxz, &r.m2_vzx};
+    for (int q = 0; q < 17; ++q)
+      r.out[q] = q < 5             ? h->fc(q, 1 - h->cur)
+                 : q < 9 || q > 12 ? h->mc(q - 5, 1 - h->cur)
+                                   : (float*)(h->base + h->L.off_memS[q - 9]);
+    for (const int64_t n = nsteps / (2 * kS2Steps) * (2 * kS2Steps); done < n; done += kS2Steps) {
+      r.t0 = (int)(h->step + done);
+      seis2_stream_launch(r, plan, h->stream);
+      for (int q = 0; q < 17; ++q) std::swap(*at[q], r.out[q]);
+    }
+  }
+  return run_steps(h, nsteps - done, (int)done);
+}
+
+// A streaming electromag2c run.  One step, and two of a large grid, are faster in
+// the two kernels of a step than in a tile's launch and the state's way back (1040 x
+// 540 cells: 31 against 46 us, 1400 x 1000 45 and 83; two steps 49 and 48, 78 and 89).
+int em2c_stream_run(sfd_handle* h, int64_t nsteps) {
+  const Layout& L = h->L;
+  if (nsteps == 1 || (nsteps == 2 && (size_t)L.P * L.NZ > 800000)) return run_steps(h, nsteps, 0);
+  StreamPlan plan;
+  CK(em2c_stream_prepare(h->cfg.nx, h->cfg.nz, h->cfg.npml, &plan));
+  const int64_t n = (nsteps + kC2Halo - 1) / kC2Halo;
+  Em2cStream r;
+  r.from = h->em2c;
+  for (int64_t l = 0; l < n; ++l) {
+    const int from = (int)(l & 1), to = 1 - from;
+    for (int q = 0; q < 2; ++q) {
+      r.from.Ex[q] = h->fc(q, from); r.from.Ez[q] = h->fc(2 + q, from); r.from.Hy[q] = h->fc(4 + q, from);
+      r.from.mExz[q] = h->mc(q, from); r.from.mEzx[q] = h->mc(2 + q, from);
+      r.from.mHyz[q] = h->mc(4 + q, from); r.from.mHyx[q] = h->mc(6 + q, from);
+      r.Ex[q] = h->fc(q, to); r.Ez[q] = h->fc(2 + q, to); r.Hy[q] = h->fc(4 + q, to);
+      r.mExz[q] = h->mc(q, to); r.mEzx[q] = h->mc(2 + q, to); r.mHyz[q] = h->mc(4 + q, to); r.mHyx[q] = h->mc(6 + q, to);
+    }
+    const int64_t s0 = nsteps * l / n, s1 = nsteps * (l + 1) / n;
+    r.t0 = (int)(h->step + s0);
+    r.nsteps = (int)(s1 - s0);
+    em2c_stream_launch(r, plan, h->stream);
+  }
+  if (n & 1) {  // back to the first copy: its fields and its memory variables lie back to back, the second's likewise
+    CK(cudaMemcpyAsync(h->fc(0, 0), h->fc(0, 1), sizeof(float) * L.fsz * 6, cudaMemcpyDeviceToDevice, h->stream));
+    CK(cudaMemcpyAsync(h->mc(0, 0), h->mc(0, 1), L.off_memB[7] - L.off_memB[0] + sizeof(float) * L.mem_sz[7],
+                       cudaMemcpyDeviceToDevice, h->stream));
+  }
+  return SFD_OK;
 }
 
 // Host rows of NX floats -> device rows of pitch P.
@@ -1554,115 +1656,20 @@ int32_t sfd_run(sfd_handle* h, int64_t nsteps) {
   if (h->step + nsteps > h->cfg.nstep)
     return fail(SFD_ERR_BAD_ARG, "run to step %lld exceeds the %d source samples", (long long)(h->step + nsteps), h->cfg.nstep);
   if (nsteps == 0) return SFD_OK;
-  const Layout& L = h->L;
-  Ctl* ctl = (Ctl*)(h->base + L.off_ctl);
-  float* slots = (float*)(h->base + L.off_slots);
   if (resident_usable(h)) return run_on_chip(h, nsteps, h->wait_ns);
   begin_run(h, h->step);
+  int rc;
   if (h->single && h->cfg.kind == SFD_ELECTROMAG2) {
-    StreamPlan plan;
-    CK(em2_stream_prepare(h->cfg.nx, h->cfg.nz, h->cfg.npml, &plan));
-    const int64_t n = stream_launches(nsteps, kTileHalo);
-    for (int64_t l = 0; l < n; ++l) {
-      const int64_t s0 = nsteps * l / n, s1 = nsteps * (l + 1) / n;
-      Em2Resident r = resident_args(h, s1 - s0);
-      const int q = 1 - h->cur;
-      r.oEx = h->fc(0, q); r.oEz = h->fc(1, q); r.oHy = h->fc(2, q);
-      r.omExz = h->mc(0, q); r.omEzx = h->mc(1, q); r.omHyz = h->mc(2, q); r.omHyx = h->mc(3, q);
-      r.t0 += (int)s0;
-      em2_stream_launch(r, plan, h->stream);
-      h->cur = q;
-    }
-    reduce_norms(h);
-    CK(cudaGetLastError());
-    h->step += nsteps;
-    return SFD_OK;
+    rc = em2_stream_run(h, nsteps);
+  } else if (streams_seis2(h->cfg)) {
+    rc = seis2_stream_run(h, nsteps);
+  } else if (streams_complex(h->cfg)) {
+    rc = em2c_stream_run(h, nsteps);
+  } else {
+    rc = run_steps(h, nsteps, 0);
   }
-  if (streams_seis2(h->cfg)) {
-    StreamPlan plan;
-    CK(seis2_stream_prepare(h->cfg.nx, h->cfg.nz, h->cfg.npml, &plan));
-    const int64_t n = (nsteps + kS2Steps - 1) / kS2Steps;
-    Seis2Resident r = seis2_resident_args(h, 0);
-    float** at[17] = {&r.vx, &r.vz, &r.sxx, &r.szz, &r.sxz, &r.m_vxx, &r.m_vzz, &r.m_vxz, &r.m_vzx, &r.m_sxx_x, &r.m_szz_z,
-                      &r.m_sxz_x, &r.m_sxz_z, &r.m2_vxx, &r.m2_vzz, &r.m2_vxz, &r.m2_vzx};
-    for (int q = 0; q < 17; ++q)
-      r.out[q] = q < 5             ? h->fc(q, 1 - h->cur)
-                 : q < 9 || q > 12 ? h->mc(q - 5, 1 - h->cur)
-                                   : (float*)(h->base + L.off_memS[q - 9]);
-    for (int64_t l = 0; l < n; ++l) {
-      const int64_t s0 = nsteps * l / n, s1 = nsteps * (l + 1) / n;
-      r.t0 = (int)(h->step + s0);
-      r.nsteps = (int)(s1 - s0);
-      seis2_stream_launch(r, plan, h->stream);
-      for (int q = 0; q < 17; ++q) std::swap(*at[q], r.out[q]);
-      h->cur ^= 1;
-    }
-    // arrays first .. last lie back to back, in every copy
-    auto copy = [&](float* dst, const float* src, int first, int last) {
-      return cudaMemcpyAsync(dst, src, L.off_mem[last] - L.off_mem[first] + sizeof(float) * L.mem_sz[last],
-                             cudaMemcpyDeviceToDevice, h->stream);
-    };
-    if (n & 1) CK(copy(h->mc(4, 0), (const float*)(h->base + L.off_memS[0]), 4, 7));  // their one copy that stays
-    if ((n ^ nsteps) & 1) {  // into the copy that one launch a step would leave the state in
-      const int p = h->cur, q = 1 - p;
-      CK(cudaMemcpyAsync(h->fc(0, q), h->fc(0, p), sizeof(float) * L.fsz * 5, cudaMemcpyDeviceToDevice, h->stream));
-      CK(copy(h->mc(0, q), h->mc(0, p), 0, 3));
-      CK(copy(h->mc(8, q), h->mc(8, p), 8, 11));
-      h->cur = q;
-    }
-    reduce_norms(h);
-    CK(cudaGetLastError());
-    h->step += nsteps;
-    return SFD_OK;
-  }
-  if (streams_complex(h->cfg)) {
-    StreamPlan plan;
-    CK(em2c_stream_prepare(h->cfg.nx, h->cfg.nz, h->cfg.npml, &plan));
-    const int64_t n = (nsteps + kC2Halo - 1) / kC2Halo;
-    Em2cStream r;
-    r.from = h->em2c;
-    for (int64_t l = 0; l < n; ++l) {
-      const int from = (int)(l & 1), to = 1 - from;
-      for (int q = 0; q < 2; ++q) {
-        r.from.Ex[q] = h->fc(q, from); r.from.Ez[q] = h->fc(2 + q, from); r.from.Hy[q] = h->fc(4 + q, from);
-        r.from.mExz[q] = h->mc(q, from); r.from.mEzx[q] = h->mc(2 + q, from);
-        r.from.mHyz[q] = h->mc(4 + q, from); r.from.mHyx[q] = h->mc(6 + q, from);
-        r.Ex[q] = h->fc(q, to); r.Ez[q] = h->fc(2 + q, to); r.Hy[q] = h->fc(4 + q, to);
-        r.mExz[q] = h->mc(q, to); r.mEzx[q] = h->mc(2 + q, to); r.mHyz[q] = h->mc(4 + q, to); r.mHyx[q] = h->mc(6 + q, to);
-      }
-      const int64_t s0 = nsteps * l / n, s1 = nsteps * (l + 1) / n;
-      r.t0 = (int)(h->step + s0);
-      r.nsteps = (int)(s1 - s0);
-      em2c_stream_launch(r, plan, h->stream);
-    }
-    if (n & 1) {  // back to the first copy: its fields and its memory variables lie back to back, the second's likewise
-      CK(cudaMemcpyAsync(h->fc(0, 0), h->fc(0, 1), sizeof(float) * L.fsz * 6, cudaMemcpyDeviceToDevice, h->stream));
-      CK(cudaMemcpyAsync(h->mc(0, 0), h->mc(0, 1), L.off_memB[7] - L.off_memB[0] + sizeof(float) * L.mem_sz[7],
-                         cudaMemcpyDeviceToDevice, h->stream));
-    }
-    reduce_norms(h);
-    CK(cudaGetLastError());
-    h->step += nsteps;
-    return SFD_OK;
-  }
-  const int64_t chunks = h->cap_stream ? nsteps / kGraphSteps : 0;
-  const int rem = (int)(nsteps - chunks * kGraphSteps);
-  if (chunks > 0) {
-    int r = ensure_graph(h, h->single ? h->cur : 0);
-    if (r) return r;
-    for (int64_t q = 0; q < chunks; ++q) CK(cudaGraphLaunch(h->graph[h->single ? h->cur : 0], h->stream));
-  }
-  for (int s = 0; s < rem; ++s) {
-    if (h->single) {
-      launch_step(h, h->cur, s, h->stream);
-      h->cur ^= 1;
-    } else {
-      launch_half(h, 0, s, h->stream);
-      launch_half(h, 1, s, h->stream);
-    }
-  }
-  launch_finalize(h, (int)(h->step + nsteps - 1), h->stream);
-  k_reduce_slots<<<1, 1024, 0, h->stream>>>(ctl, slots, L.nslots);
+  if (rc) return rc;
+  reduce_norms(h);
   CK(cudaGetLastError());
   h->step += nsteps;
   return SFD_OK;

@@ -54,6 +54,7 @@ struct Em2cArgs {
   AxisTab X, Z;
   float dbH;
   IoArgs io;  // source rows and trace channels: Ex re, Ex im, Ez re, Ez im
+  int as_tiles;  // the two kernels round as the streaming tiles do
 };
 
 struct Seis2Args {

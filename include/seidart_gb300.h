@@ -432,19 +432,28 @@ int32_t sfd_adjoint_gradient(sfd_handle* h, double* planes, int64_t count);
  * Many 2-D models (electromag2 shots, seismic2 models of any sizes, mixed)
  * advance by one call.  Models that are faster alone on chip run so, one
  * after another; the others advance together in one persistent cooperative
- * kernel launch with a grid barrier per time step.  Replaces the per-shot process loop of the driver
- * (src/seidart/simulations/common_offset.py:143-284, one seidartfdtd call per
- * source).  The handles must be single-pass 2-D handles on one stream with
+ * kernel launch with a grid barrier per time step.  Which ones depends on the
+ * run's length and on the models, their results do not: either way gives a
+ * model the bits of its own run.  Replaces the per-shot process loop of the
+ * driver (src/seidart/simulations/common_offset.py:143-284, one seidartfdtd
+ * call per source).  The handles must be single-pass 2-D handles on one stream with
  * model and CPML set; each keeps its own state, source, receivers and traces.
  * The batch needs a small device scratch buffer of sfd_batch_scratch_bytes. */
 typedef struct sfd_batch_s sfd_batch;
 int32_t sfd_batch_scratch_bytes(int32_t nmodels, size_t* bytes);
 int32_t sfd_batch_create(sfd_handle* const* handles, int32_t nmodels, void* dev_scratch, size_t bytes,
                          sfd_batch** out);
-/* Tile rows per thread (1, 2, 4) and resident blocks per SM of the launch. */
+/* Tile rows per thread (1, 2, 4) and resident blocks per SM of the persistent
+ * launch; the models that run on chip have tilings of their own. */
 int32_t sfd_batch_set_tiling(sfd_batch* b, int32_t zb, int32_t blocks_per_sm);
 /* Advance every model nsteps steps (asynchronous). */
 int32_t sfd_batch_run(sfd_batch* b, int64_t nsteps);
+/* How many models a run of nsteps steps advances on chip, each alone. */
+int32_t sfd_batch_on_chip(sfd_batch* b, int64_t nsteps, int32_t* count);
+/* Tuning aid: nsteps steps, in the persistent launch, of the models that a run of
+ * all their source samples advances there (of every model, when that run would
+ * advance them all on chip).  The others stay; reset the models afterwards. */
+int32_t sfd_batch_trial(sfd_batch* b, int64_t nsteps);
 /* Longest wait, in ns, of a block at the batch kernel's grid barrier; 0
  * restores the default, 2 s.  A wait that runs out makes every block leave
  * the kernel and sfd_batch_status return SFD_ERR_TIMEOUT. */

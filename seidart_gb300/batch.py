@@ -36,6 +36,8 @@ def _declare(L):
         ("sfd_batch_create", i32, [C.POINTER(P), i32, P, sz, C.POINTER(P)]),
         ("sfd_batch_set_tiling", i32, [P, i32, i32]),
         ("sfd_batch_run", i32, [P, i64]),
+        ("sfd_batch_on_chip", i32, [P, i64, C.POINTER(i32)]),
+        ("sfd_batch_trial", i32, [P, i64]),
         ("sfd_batch_status", i32, [P, C.POINTER(i32)]),
         ("sfd_batch_set_wait_limit", i32, [P, i64]),
         ("sfd_batch_test_stall_waits", i32, [P, i32]),
@@ -74,11 +76,25 @@ class Batch:
         return sum(s.grid.cells for s in self.solvers)
 
     def set_tiling(self, zb: int, blocks_per_sm: int) -> None:
+        """Rows per thread and blocks per SM of the persistent launch (models
+        that run on chip have tilings of their own)."""
         check(self._L.sfd_batch_set_tiling(self._b, int(zb), int(blocks_per_sm)))
         self.tiling = (int(zb), int(blocks_per_sm))
 
     def run(self, nsteps: int) -> None:
         check(self._L.sfd_batch_run(self._b, int(nsteps)))
+
+    def on_chip(self, nsteps: int) -> int:
+        """How many models a run of ``nsteps`` steps advances on chip, each alone."""
+        n = C.c_int32()
+        check(self._L.sfd_batch_on_chip(self._b, int(nsteps), C.byref(n)))
+        return n.value
+
+    def trial(self, nsteps: int) -> None:
+        """Tuning aid: ``nsteps`` steps, in the persistent launch, of the models
+        that a whole run advances there (of every model, when it would advance
+        them all on chip); the others stay."""
+        check(self._L.sfd_batch_trial(self._b, int(nsteps)))
 
     def set_wait_limit(self, ns: int) -> None:
         """Longest wait (ns) at the kernel's grid barrier; 0 = the default 2 s."""
@@ -101,6 +117,9 @@ class Batch:
         import torch
         dev = torch.cuda.get_device_name(self.solvers[0].device)
         key = [dev] + [f"{s.kind}:{s.grid.nx}x{s.grid.nz}" for s in self.solvers]
+        alone = self.on_chip(min(s.nstep for s in self.solvers))
+        if alone:  # the tiling is that of the others
+            key.append(f"{alone} on chip")
         return hashlib.sha1("|".join(key).encode()).hexdigest()[:16]
 
     def close(self) -> None:
@@ -120,7 +139,8 @@ def _cache_path() -> Path:
 
 
 def autotune(batch: Batch, steps: int = 16, candidates=CANDIDATES, use_cache: bool = True, verbose: bool = False):
-    """Time each (rows per thread, blocks per SM) candidate for ``steps`` steps
+    """Time each (rows per thread, blocks per SM) candidate of the persistent
+    launch for ``steps`` steps of the models that a whole run advances in it,
     and keep the fastest.  The trial steps advance the models, so every
     solver is reset afterwards: call this before the real run."""
     import torch
@@ -145,11 +165,11 @@ def autotune(batch: Batch, steps: int = 16, candidates=CANDIDATES, use_cache: bo
         except _lib.SfdError:
             continue
         batch.reset()
-        batch.run(2)
+        batch.trial(2)
         batch.status()
         torch.cuda.synchronize()
         t0 = time.perf_counter()
-        batch.run(steps)
+        batch.trial(steps)
         batch.status()
         el = (time.perf_counter() - t0) / steps
         timings[f"{zb}x{bps}"] = el

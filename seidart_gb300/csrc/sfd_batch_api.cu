@@ -76,6 +76,17 @@ std::vector<char> choose_on_chip(const std::vector<sfd_handle*>& h, int64_t nste
     for (int m = 0; m < n; ++m) alone[m] = fits[m];
   return alone;
 }
+
+// Whether nsteps more steps of every model of the batch can run.
+int check_run(const sfd_batch_s* b, int64_t nsteps) {
+  if (!b) return fail(SFD_ERR_BAD_ARG, "NULL batch");
+  if (nsteps < 0) return fail(SFD_ERR_BAD_ARG, "nsteps must be >= 0");
+  for (size_t m = 0; m < b->h.size() && nsteps > 0; ++m)
+    if (b->h[m]->step + nsteps > b->h[m]->cfg.nstep)
+      return fail(SFD_ERR_BAD_ARG, "model %d: run to step %lld exceeds its %d source samples", (int)m,
+                  (long long)(b->h[m]->step + nsteps), b->h[m]->cfg.nstep);
+  return SFD_OK;
+}
 }  // namespace
 
 extern "C" {
@@ -127,16 +138,35 @@ int32_t sfd_batch_set_tiling(sfd_batch* b, int32_t zb, int32_t blocks_per_sm) {
   return SFD_OK;
 }
 
+int32_t sfd_batch_on_chip(sfd_batch* b, int64_t nsteps, int32_t* count) {
+  g_err.clear();
+  if (!b || !count) return fail(SFD_ERR_BAD_ARG, "NULL batch or count");
+  const std::vector<char> alone = choose_on_chip(b->h, nsteps);
+  *count = (int32_t)std::count(alone.begin(), alone.end(), 1);
+  return SFD_OK;
+}
+
+int32_t sfd_batch_trial(sfd_batch* b, int64_t nsteps) {
+  g_err.clear();
+  const int r = check_run(b, nsteps);
+  if (r || nsteps == 0) return r;
+  int64_t whole = b->h[0]->cfg.nstep;
+  for (const sfd_handle* h : b->h) whole = std::min<int64_t>(whole, h->cfg.nstep);
+  const std::vector<char> alone = choose_on_chip(b->h, whole);
+  std::vector<sfd_handle*> rest;
+  for (size_t m = 0; m < b->h.size(); ++m)
+    if (!alone[m]) rest.push_back(b->h[m]);
+  if (rest.empty()) rest = b->h;
+  for (sfd_handle* h : rest) h->adj_rec_n = 0;
+  CK(cudaMemsetAsync(b->bar(), 0, sizeof(GridBarrier), b->stream));
+  return run_together(b, rest, nsteps);
+}
+
 int32_t sfd_batch_run(sfd_batch* b, int64_t nsteps) {
   g_err.clear();
-  if (!b) return fail(SFD_ERR_BAD_ARG, "NULL batch");
-  if (nsteps < 0) return fail(SFD_ERR_BAD_ARG, "nsteps must be >= 0");
-  if (nsteps == 0) return SFD_OK;
+  const int rc = check_run(b, nsteps);
+  if (rc || nsteps == 0) return rc;
   const int n = (int)b->h.size();
-  for (int m = 0; m < n; ++m)
-    if (b->h[m]->step + nsteps > b->h[m]->cfg.nstep)
-      return fail(SFD_ERR_BAD_ARG, "model %d: run to step %lld exceeds its %d source samples", m,
-                  (long long)(b->h[m]->step + nsteps), b->h[m]->cfg.nstep);
   CK(cudaMemsetAsync(b->bar(), 0, sizeof(GridBarrier), b->stream));
   std::vector<sfd_handle*> rest;  // the models of the persistent launch
   const std::vector<char> alone = b->stall ? std::vector<char>(n, 0) : choose_on_chip(b->h, nsteps);

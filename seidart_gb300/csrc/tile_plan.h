@@ -64,17 +64,26 @@ bool plan_tiles(const TileRules& t, int NX, int NZ, int W, int max_ctas, size_t 
     int n = 0, z = 0;
     if (cuts) cuts->assign(1, 0);
     while (z < NZ) {
-      // the deepest band that fits, by bisection: rows, cost and memory grow with it
-      int z1 = z, over = std::min(NZ, z + max_rows) + 1;
-      while (over - z1 > 1) {
-        const int m = (z1 + over) / 2;
+      auto fits = [&](int m) {
         const Frame f = frame(c, z, m);
         const double cost = (f.rows + t.zrow * (f.zlo + f.zhi)) * (f.xlanes ? 1.0 + t.xcol : 1.0);
-        (cost > C || f.rows > max_rows || smem(f, t.max_rb) > max_smem ? over : z1) = m;
+        return cost <= C && f.rows <= max_rows && smem(f, t.max_rb) <= max_smem;
+      };
+      // the deepest band that fits.  Rows, cost and memory grow with it as long as
+      // it has its whole halo below; the last one, whose frame ends with the grid,
+      // takes less memory than those that end a few rows higher.  So: the rest of the
+      // column, or by bisection a band that leaves the last one no thinner than its
+      // neighbours' halo.
+      int z1 = NZ;
+      if (!fits(NZ)) {
+        int over = std::min(std::max(NZ - t.halo, z), z + max_rows) + 1;
+        z1 = z;
+        while (over - z1 > 1) {
+          const int m = (z1 + over) / 2;
+          (fits(m) ? z1 : over) = m;
+        }
       }
       if (z1 == z) return max_ctas + 1;
-      // a last band of a few rows: no thinner than its neighbours' halo
-      if (NZ - z1 > 0 && NZ - z1 < t.halo) z1 = std::max(z + 1, NZ - t.halo);
       z = z1;
       ++n;
       if (cuts) cuts->push_back(z);

@@ -968,7 +968,7 @@ int ensure_model_planes(sfd_handle* h) {
   parallel_for(N2, [&](size_t b, size_t e) {
     for (size_t n = b; n < e; ++n)
       for (int q = 0; q < np; ++q) model[(size_t)q * N2 + n] = t[(size_t)ids[n] * np + q];
-  });
+  }, kHostGrain);
   h->model = std::move(model);
   for (int q = 0; q < 4; ++q) h->src_plane[q] = src_full_plane(h->cfg.kind, q);  // all planes kept
   return SFD_OK;

@@ -38,10 +38,10 @@ namespace {
 // addresses and single-word accesses of every plane -- and staged 1.9 words for a
 // word of a neighbouring field.  Four columns a thread share the first and move
 // 16 bytes an access (65 instructions a cell); the one-sided halo of 32 x 16
-// columns stages 1.2 words: 106 + 132 us, 0.248 against 0.299 ms a step.  What is
+// columns stages 1.2 words: 107 + 135 us, 0.252 against 0.299 ms a step.  What is
 // left is the latency of a plane's chain at 12 warps an SM: rings of 3 and 5
-// planes (16 and 8 warps) run 0.257 and 0.268 ms, blocks of 8 rows 0.249.  The x
-// and z strips' variables, loaded where they were used, cost 0.325 ms.
+// planes (16 and 8 warps) ran 0.009 and 0.020 ms longer, blocks of 8 rows 0.001.  The
+// x and z strips' variables, loaded where they were used, cost 0.077 ms.
 constexpr int BX = 32;
 constexpr int VW = BX + 4;  // floats of a staged row with its halo
 constexpr int kRing = 4;  // staged planes per block

@@ -1,12 +1,14 @@
-// SM-resident 2-D time stepping: a whole run in one cooperative launch, with
-// every tile's fields, coefficients and memory variables held in shared
-// memory for all of its steps.
+// SM-resident 2-D time stepping: a whole run in one cooperative launch, every
+// tile's state held in registers and shared memory for all of its steps, one CTA
+// per tile and at most one CTA per SM.  Global memory holds the state only before
+// and after the run, and the words through which tiles exchange what their
+// neighbours need; a word carries its tag, which is the only synchronisation
+// between tiles.
 //
-// The grid is cut into ntx x ntz tiles of TW x TZ cells, one CTA per tile and
-// at most one CTA per SM.  Per step a CTA exchanges only its one-cell edges
-// with its neighbours, through small edge arrays in global memory (L2); the
-// edge words carry their step, which is the only synchronisation between
-// tiles.  Global memory holds the state only before and after the run.
+// Runs of the tiles of several steps (em2_run.cuh, s2_run.cuh) hand over halos of
+// four cells every four or two steps.  The electromag2 adjoint sweep
+// (resident_adj.cu) and the seismic2 run with the legacy quirks
+// (resident_s2_legacy.cu) exchange one-cell edges twice a step.
 #pragma once
 #include <cuda_runtime.h>
 #include "sfd_solvers.h"

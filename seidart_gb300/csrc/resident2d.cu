@@ -20,17 +20,17 @@
 // What bounds it: the chain of a step -- two block barriers, a row of shared
 // memory each way, about 60 instructions for each row of four cells -- and,
 // every fourth step, the hand-over through L2.  On 1040 x 540 cells a step
-// takes 1.81 us (1.3 us of it the step of the largest tiles, the rest a
-// hand-over of 2.2 us in four); 120 x 90 cells take 1.3 us.  The form before
+// takes 1.83 us (1.3 us of it the step of the largest tiles, the rest a
+// hand-over of 2.2 us in four); 120 x 90 cells take 1.2 to 1.3 us.  The form before
 // it exchanged one-cell edges twice a step, every cell mask applied in the
 // step: 4.24 and 4.3 us.
 //
 // The per-cell arithmetic is that of the loops of
 // legacy/fortran/electromagfdtd.f95:249-321.  Every product and sum names its
 // rounding, so that a cell gets the same bits from whichever tile computes it
-// (its own or one whose halo it lies in) and whichever form of the kernel: a
-// run in pieces, with checkpoints or recomputed for the adjoint gives the
-// states of the plain run.
+// (its own or one whose halo it lies in) and whichever form of the kernel, here,
+// streamed, one step a launch or batched: a run in pieces, with checkpoints or
+// recomputed for the adjoint gives the states of the plain run.
 #include <algorithm>
 
 #include "em2_run.cuh"

@@ -731,9 +731,9 @@ int run_steps(sfd_handle* h, int64_t nsteps, int done) {
 // single steps.  Each launch goes from one copy of the state to the other, and so
 // many of them are of their steps' parity: the state ends in the copy that one
 // launch a step would leave it in.  (4040 x 3040 cells, us a run of 1, 2, 4, 5, 7
-// steps, set-up and norms included: 138, 245, 294, 399, 449; in the fewest launches
+// steps, set-up and norms included: 136, 239, 299, 402, 460; in the fewest launches
 // of that parity, single steps among them as launches of one, 165, 301, 325, 461,
-// 486.  300 x 200 cells: 19, 27, 33, 41, 43 and 22, 39, 41, 57, 60.)
+// 486.  300 x 200 cells: 21, 29, 39, 48, 58 and 22, 39, 41, 57, 60.)
 int em2_stream_run(sfd_handle* h, int64_t nsteps) {
   StreamPlan plan;
   int64_t done = 0;
@@ -755,7 +755,7 @@ int em2_stream_run(sfd_handle* h, int64_t nsteps) {
 
 // A streaming seismic2 run: launches of two steps in pairs, so that the state ends
 // in the copy that one launch a step would leave it in, then single steps.  (2040 x
-// 1540 cells, us a run of 1, 2, 3, 5 steps: 103, 188, 274, 397; in launches of two
+// 1540 cells, us a run of 1, 2, 3, 5 steps: 103, 188, 273, 388; in launches of two
 // and one with the state copied back 151, 199, 322, 434.)
 int seis2_stream_run(sfd_handle* h, int64_t nsteps) {
   StreamPlan plan;

@@ -51,7 +51,7 @@ bool same_group(const sfd_handle* a, const sfd_handle* b) {
 // cells and 18 for a million seismic2 cells; a model alone on chip 1.1 + 1.3
 // and 1.9 + 4 for a million cells, and 20 a run.  (Eight 1040 x 540 shots and
 // four elastic models of 126,000 to 185,000 cells took 107 a step in the
-// persistent launch and 24 one after another; 32 shots of 120 x 90 cells 23
+// persistent launch and 27 one after another; 32 shots of 120 x 90 cells 23
 // and 34.)
 std::vector<char> choose_on_chip(const std::vector<sfd_handle*>& h, int64_t nsteps) {
   const int n = (int)h.size();

@@ -70,10 +70,10 @@ size_t tile_smem(int NX, int NZ, int W, int rb, int ntx, int nbz) {
 
 // Tiles are worth it where they fill 0.7 of their waves (one CTA an SM): a launch of
 // one wave takes 23 us, of two 32, of three 43, whatever the last one holds, and a
-// single-pass step 7 us and 20 for a million cells.  (us a step so and so: 635 x 460
-// cells, 0.86 of one wave, 11.5 and 12.6; 723 x 549, 0.58 of two, 15.9 and 15.3;
-// 1036 x 501, 0.76 of two, 15.7 and 17.7; 897 x 907, 0.80 of three, 21.4 and 22.7.)
-// Grids of less than a wave run here only when told to stream.
+// single-pass step 7 us and 20 for a million cells.  (us a step so and so: 440 x 240
+// cells, 0.31 of one wave, 11.5 and 8.2; 635 x 460, 0.86, 11.5 and 12.6; 723 x 549,
+// 0.58 of two, 15.9 and 15.3; 1036 x 501, 0.76 of two, 15.7 and 17.7; 897 x 907,
+// 0.80 of three, 21.4 and 22.7.)
 constexpr double kWorth = 0.7;
 
 cudaError_t seis2_stream_prepare(int NX, int NZ, int W, StreamPlan* out, bool* faster) {
@@ -93,7 +93,7 @@ cudaError_t seis2_stream_prepare(int NX, int NZ, int W, StreamPlan* out, bool* f
   }
   const int waves = (out->ntx * out->nbz + sms - 1) / sms;
   const double wave = (double)sms * (kSC - 2 * kS2Halo) * (kS2Warps * out->rb - 2 * kS2Halo);  // cells
-  *faster = waves == 1 || (double)NX * NZ > kWorth * waves * wave;
+  *faster = (double)NX * NZ > kWorth * waves * wave;
   return res_allow_max_smem((const void*)kernel_of(out->rb));
 }
 

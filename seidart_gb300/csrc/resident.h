@@ -76,11 +76,12 @@ constexpr int kS2MaxRows = 3;
 inline size_t s2_word_bytes(int P, int NZ, int W) {
   return 2 * sizeof(uint4) * 2 * ((size_t)NZ * P + 2 * (size_t)W * P + (size_t)NZ * 2 * W);
 }
-constexpr size_t kS2MaxCells = (size_t)kResMaxTiles * 60 * kS2MaxRows * 16;
+// Largest grids (cells of pitch) that may run on chip: a whole frame for each of a
+// GB300's SMs (152, of 160 on the dies).  Larger ones get no hand-over words.
+constexpr size_t kMostSms = 160;
+constexpr size_t kS2MaxCells = kMostSms * 64 * kS2MaxRows * 16;
+constexpr size_t kEm2MaxCells = kMostSms * 128 * kEm2MaxRows * kEm2MaxWarps;
 __host__ __device__ inline int s2_hand_overs(int nsteps) { return nsteps <= kS2Steps ? 1 : (nsteps - 1) / kS2Steps; }
-// Largest grid (cells of pitch) an electromag2 run can hold on chip; larger
-// ones get no hand-over words.
-constexpr size_t kEm2MaxCells = (size_t)kResMaxTiles * 124 * kEm2MaxRows * kEm2MaxWarps;
 // Hand-overs of a run of nsteps steps: after every kTileHalo-th but the last;
 // a run of no more steps has one before its first.
 __host__ __device__ inline int em2_hand_overs(int nsteps) {

@@ -472,7 +472,7 @@ __device__ __forceinline__ void em2_run_tile(const Em2Resident& a, Em2Tile& G, i
         }
         // dEz/dx, rounded or fused into the sum (em2_rounded; where it is fused, p is
         // zero).  A select: two forms of the loop, or a branch a row, cost 4 to 7 %
-        // of a step of 1040 x 540 cells, this 1 %; the mask alone costs frames of two
+        // of a step of 1040 x 540 cells, this 1 to 3 %; the mask alone costs frames of two
         // and four rows a warp 1 to 4 % more, the other way those of one and three.
         const bool round = RB & 1 ? roundall >> j & 1u : roundx || (rounded >> j & 1u);
 #pragma unroll

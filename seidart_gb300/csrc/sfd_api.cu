@@ -764,9 +764,11 @@ int seis2_stream_run(sfd_handle* h, int64_t nsteps) {
   if (tiles) CK(seis2_stream_prepare(h->cfg.nx, h->cfg.nz, h->cfg.npml, &plan, &tiles));
   // single steps are faster by graph only (16 of 723 x 549 cells one by one 284 us, in
   // tiles 257), and a graph launch would end a capture of the caller's stream
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  CK(cudaStreamIsCapturing(h->stream, &capture));
-  tiles = nsteps >= 2 * kS2Steps && (tiles || nsteps < kGraphSteps || capture != cudaStreamCaptureStatusNone);
+  if (nsteps >= 2 * kS2Steps && !tiles) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(h->stream, &capture) != cudaSuccess) cudaGetLastError();
+    tiles = nsteps < kGraphSteps || capture != cudaStreamCaptureStatusNone;
+  }
   if (tiles) {
     Seis2Resident r = seis2_resident_args(h, kS2Steps);
     float** at[17] = {&r.vx, &r.vz, &r.sxx, &r.szz, &r.sxz, &r.m_vxx, &r.m_vzz, &r.m_vxz, &r.m_vzx, &r.m_sxx_x, &r.m_szz_z,
